@@ -9,7 +9,7 @@
 //   paged_attention_v1              ops.h:6       (attention/attention_kernels.cu)
 // Layouts are this library's own: the KV cache is [num_blocks, block_size, kv_heads, 128] for K
 // and for V (one 256-byte row per token and head), head size 128 only (every Llama-2 size).
-#include "dz_elem.cuh"
+#include "dz_grouped_decode.cuh"
 
 namespace dz {
 namespace {
@@ -167,11 +167,11 @@ rotary_cache_kernel(T* __restrict__ qkv, const int64_t* __restrict__ positions,
 
 // ---------------------------------------------------------------------------
 // Decode attention over the paged cache: one query token per sequence.
-// Grid (kv_heads, sequences, splits); a CTA handles the G = q_heads / kv_heads query heads that
-// share one kv head, over the key range of its split, so K and V are read once.  The warps take
-// the rows of the range in turn (how the lanes share a row depends on G, see the two forms
-// below), scores are reduced with shuffles, softmax is computed online and the warps' partial
-// (max, sum, acc) are merged through shared memory.
+// Grid (kv_heads, sequences, splits); a CTA handles the G = q_heads / kv_heads query heads (one or
+// two; more go to dz_grouped_decode.cu) that share one kv head, over the key range of its split,
+// so K and V are read once.  The warps take the rows of the range in turn, scores are reduced
+// with shuffles, softmax is computed online and the warps' partial (max, sum, acc) are merged
+// through shared memory.
 // With splits > 1 the CTA writes its partial triple to `partial` and the last CTA of a
 // (sequence, kv head) to arrive -- counted with an atomic ticket -- merges the splits; nothing
 // waits on anything.
@@ -198,160 +198,94 @@ paged_decode_attention_kernel(const T* __restrict__ qkv, int q_row_stride, T* __
   const int q_heads = kv_heads * G;
 
   const int* table = block_tables + (size_t)seq * max_blocks;
-  if constexpr (G <= 2) {
-    // Few query heads per key/value head: the kernel is a pure stream of K and V rows, so what
-    // counts is bytes in flight.  A half-warp owns a row (16 lanes x 16 bytes), a warp two rows
-    // per load instruction, and two such pairs are requested per iteration: 64 bytes in flight
-    // per lane.  Each half-warp keeps its own running (max, sum, accumulator); the halves are
-    // merged by shuffles at the end, the warps through shared memory as in the general form.
-    const int half = lane >> 4, hl = lane & 15;
-    float q[G][8];
+  // Few query heads per key/value head: the kernel is a pure stream of K and V rows, so what
+  // counts is bytes in flight.  A half-warp owns a row (16 lanes x 16 bytes), a warp two rows
+  // per load instruction, and two such pairs are requested per iteration: 64 bytes in flight
+  // per lane.  Each half-warp keeps its own running (max, sum, accumulator); the halves are
+  // merged by shuffles at the end, the warps through shared memory as in the general form.
+  const int half = lane >> 4, hl = lane & 15;
+  float q[G][8];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const uint4 v = *reinterpret_cast<const uint4*>(qkv + (size_t)seq * q_row_stride +
-                                                      (size_t)(kh * G + g) * kHeadDim + hl * 8);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (int g = 0; g < G; ++g) {
+    const uint4 v = *reinterpret_cast<const uint4*>(qkv + (size_t)seq * q_row_stride +
+                                                    (size_t)(kh * G + g) * kHeadDim + hl * 8);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = Cvt<T>::up(w[j]);
+      q[g][2 * j] = f.x * scale;
+      q[g][2 * j + 1] = f.y * scale;
+    }
+  }
+  float m[G], l[G], acc[G][8];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    m[g] = -INFINITY; l[g] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[g][j] = 0.f;
+  }
+  for (int base = t0 + 2 * warp; base < t1; base += 4 * kWarps) {
+    const int ta = base + half, tb = ta + 2 * kWarps;
+    const bool va_ok = ta < t1, vb_ok = tb < t1;
+    const int tac = min(ta, t1 - 1), tbc = min(tb, t1 - 1);     // rows read for absent tokens
+    const size_t ra = ((size_t)table[tac / block_size] * block_size + tac % block_size) * kv_heads + kh;
+    const size_t rb = ((size_t)table[tbc / block_size] * block_size + tbc % block_size) * kv_heads + kh;
+    const uint4 ka = *reinterpret_cast<const uint4*>(k_cache + ra * kHeadDim + hl * 8);
+    const uint4 kb = *reinterpret_cast<const uint4*>(k_cache + rb * kHeadDim + hl * 8);
+    const uint4 va = *reinterpret_cast<const uint4*>(v_cache + ra * kHeadDim + hl * 8);
+    const uint4 vb = *reinterpret_cast<const uint4*>(v_cache + rb * kHeadDim + hl * 8);
+    float fka[8], fkb[8], fva[8], fvb[8];
+    {
+      const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb.x, kb.y, kb.z, kb.w};
+      const uint32_t xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 f = Cvt<T>::up(w[j]);
-        q[g][2 * j] = f.x * scale;
-        q[g][2 * j + 1] = f.y * scale;
+        float2 f = Cvt<T>::up(wa[j]); fka[2 * j] = f.x; fka[2 * j + 1] = f.y;
+        f = Cvt<T>::up(wb[j]); fkb[2 * j] = f.x; fkb[2 * j + 1] = f.y;
+        f = Cvt<T>::up(xa[j]); fva[2 * j] = f.x; fva[2 * j + 1] = f.y;
+        f = Cvt<T>::up(xb[j]); fvb[2 * j] = f.x; fvb[2 * j + 1] = f.y;
       }
     }
-    float m[G], l[G], acc[G][8];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      m[g] = -INFINITY; l[g] = 0.f;
+      float sa = 0.f, sb = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[g][j] = 0.f;
-    }
-    for (int base = t0 + 2 * warp; base < t1; base += 4 * kWarps) {
-      const int ta = base + half, tb = ta + 2 * kWarps;
-      const bool va_ok = ta < t1, vb_ok = tb < t1;
-      const int tac = min(ta, t1 - 1), tbc = min(tb, t1 - 1);     // rows read for absent tokens
-      const size_t ra = ((size_t)table[tac / block_size] * block_size + tac % block_size) * kv_heads + kh;
-      const size_t rb = ((size_t)table[tbc / block_size] * block_size + tbc % block_size) * kv_heads + kh;
-      const uint4 ka = *reinterpret_cast<const uint4*>(k_cache + ra * kHeadDim + hl * 8);
-      const uint4 kb = *reinterpret_cast<const uint4*>(k_cache + rb * kHeadDim + hl * 8);
-      const uint4 va = *reinterpret_cast<const uint4*>(v_cache + ra * kHeadDim + hl * 8);
-      const uint4 vb = *reinterpret_cast<const uint4*>(v_cache + rb * kHeadDim + hl * 8);
-      float fka[8], fkb[8], fva[8], fvb[8];
-      {
-        const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb.x, kb.y, kb.z, kb.w};
-        const uint32_t xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
+      for (int j = 0; j < 8; ++j) { sa += q[g][j] * fka[j]; sb += q[g][j] * fkb[j]; }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 f = Cvt<T>::up(wa[j]); fka[2 * j] = f.x; fka[2 * j + 1] = f.y;
-          f = Cvt<T>::up(wb[j]); fkb[2 * j] = f.x; fkb[2 * j + 1] = f.y;
-          f = Cvt<T>::up(xa[j]); fva[2 * j] = f.x; fva[2 * j + 1] = f.y;
-          f = Cvt<T>::up(xb[j]); fvb[2 * j] = f.x; fvb[2 * j + 1] = f.y;
-        }
+      for (int o = 8; o > 0; o >>= 1) {            // within the half-warp
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        sb += __shfl_xor_sync(0xffffffffu, sb, o);
       }
+      if (va_ok) {                                  // vb_ok implies va_ok
+        if (!vb_ok) sb = -INFINITY;
+        const float mn = fmaxf(m[g], fmaxf(sa, sb));
+        const float c = __expf(m[g] - mn), pa = __expf(sa - mn), pb = __expf(sb - mn);
+        l[g] = l[g] * c + pa + pb;
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float sa = 0.f, sb = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { sa += q[g][j] * fka[j]; sb += q[g][j] * fkb[j]; }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {            // within the half-warp
-          sa += __shfl_xor_sync(0xffffffffu, sa, o);
-          sb += __shfl_xor_sync(0xffffffffu, sb, o);
-        }
-        if (va_ok) {                                  // vb_ok implies va_ok
-          if (!vb_ok) sb = -INFINITY;
-          const float mn = fmaxf(m[g], fmaxf(sa, sb));
-          const float c = __expf(m[g] - mn), pa = __expf(sa - mn), pb = __expf(sb - mn);
-          l[g] = l[g] * c + pa + pb;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[g][j] = acc[g][j] * c + pa * fva[j] + pb * fvb[j];
-          m[g] = mn;
-        }
+        for (int j = 0; j < 8; ++j) acc[g][j] = acc[g][j] * c + pa * fva[j] + pb * fvb[j];
+        m[g] = mn;
       }
     }
-    // merge the two half-warps, then hand the warp's state to shared memory
+  }
+  // merge the two half-warps, then hand the warp's state to shared memory
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const float mo = __shfl_xor_sync(0xffffffffu, m[g], 16);
-      const float lo = __shfl_xor_sync(0xffffffffu, l[g], 16);
-      const float mm = fmaxf(m[g], mo);
-      const float c0 = (m[g] == -INFINITY) ? 0.f : __expf(m[g] - mm);
-      const float c1 = (mo == -INFINITY) ? 0.f : __expf(mo - mm);
-      const float ll = l[g] * c0 + lo * c1;
+  for (int g = 0; g < G; ++g) {
+    const float mo = __shfl_xor_sync(0xffffffffu, m[g], 16);
+    const float lo = __shfl_xor_sync(0xffffffffu, l[g], 16);
+    const float mm = fmaxf(m[g], mo);
+    const float c0 = (m[g] == -INFINITY) ? 0.f : __expf(m[g] - mm);
+    const float c1 = (mo == -INFINITY) ? 0.f : __expf(mo - mm);
+    const float ll = l[g] * c0 + lo * c1;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float ao = __shfl_xor_sync(0xffffffffu, acc[g][j], 16);
-        acc[g][j] = acc[g][j] * c0 + ao * c1;
-      }
-      if (lane == 0) { s_m[warp][g] = mm; s_l[warp][g] = ll; }
-      if (half == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s_acc[warp][g][hl * 8 + j] = acc[g][j];
-      }
+    for (int j = 0; j < 8; ++j) {
+      const float ao = __shfl_xor_sync(0xffffffffu, acc[g][j], 16);
+      acc[g][j] = acc[g][j] * c0 + ao * c1;
     }
-  } else {
-    // Grouped queries (4 or 8 query heads per kv head): lane -> (head g, part of the row), LPH =
-    // 32 / G lanes per head, each with 128 / LPH = 4 G dims of q and of the accumulator.  A warp
-    // takes one key/value row per step; the lanes of all heads read the same bytes of it (the
-    // loads coalesce into one row), a score needs log2(LPH) shuffles instead of five per head,
-    // and the K and V loads of a step are in flight together.
-    constexpr int LPH = 32 / G, DPL = 4 * G, NV = DPL / 8;     // NV 16-byte loads per row part
-    const int g = lane / LPH, part = lane % LPH;
-    float q[DPL], acc[DPL];
-    {
-      const T* qp = qkv + (size_t)seq * q_row_stride + (size_t)(kh * G + g) * kHeadDim + part * DPL;
+    if (lane == 0) { s_m[warp][g] = mm; s_l[warp][g] = ll; }
+    if (half == 0) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const uint4 u = *reinterpret_cast<const uint4*>(qp + v * 8);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = Cvt<T>::up(w[j]);
-          q[v * 8 + 2 * j] = f.x * scale;
-          q[v * 8 + 2 * j + 1] = f.y * scale;
-        }
-      }
+      for (int j = 0; j < 8; ++j) s_acc[warp][g][hl * 8 + j] = acc[g][j];
     }
-#pragma unroll
-    for (int j = 0; j < DPL; ++j) acc[j] = 0.f;
-    float m = -INFINITY, l = 0.f;
-    for (int t = t0 + warp; t < t1; t += kWarps) {
-      const size_t r = ((size_t)table[t / block_size] * block_size + t % block_size) * kv_heads + kh;
-      uint4 kk[NV], vv[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        kk[v] = *reinterpret_cast<const uint4*>(k_cache + r * kHeadDim + part * DPL + v * 8);
-        vv[v] = *reinterpret_cast<const uint4*>(v_cache + r * kHeadDim + part * DPL + v * 8);
-      }
-      float sc = 0.f;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const uint32_t w[4] = {kk[v].x, kk[v].y, kk[v].z, kk[v].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = Cvt<T>::up(w[j]);
-          sc += q[v * 8 + 2 * j] * f.x + q[v * 8 + 2 * j + 1] * f.y;
-        }
-      }
-#pragma unroll
-      for (int o = LPH / 2; o > 0; o >>= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
-      const float mn = fmaxf(m, sc);
-      const float c = __expf(m - mn), pw = __expf(sc - mn);
-      l = l * c + pw;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const uint32_t w[4] = {vv[v].x, vv[v].y, vv[v].z, vv[v].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = Cvt<T>::up(w[j]);
-          acc[v * 8 + 2 * j] = acc[v * 8 + 2 * j] * c + pw * f.x;
-          acc[v * 8 + 2 * j + 1] = acc[v * 8 + 2 * j + 1] * c + pw * f.y;
-        }
-      }
-      m = mn;
-    }
-    if (part == 0) { s_m[warp][g] = m; s_l[warp][g] = l; }
-#pragma unroll
-    for (int j = 0; j < DPL; ++j) s_acc[warp][g][part * DPL + j] = acc[j];
   }
   __syncthreads();
   // thread (g, d) pairs: G * 128 values, 256 threads
@@ -414,8 +348,6 @@ int attention_dispatch(int group, dim3 grid, cudaStream_t st, const T* qkv, int 
   switch (group) {
     case 1: DZ_CUDA_OK(launch_pdl(paged_decode_attention_kernel<T, 1>, grid, dim3(256), st, qkv, q_row_stride, out, kc, vc, bt, max_blocks, sl, block_size, kv_heads, scale, splits, partial, tickets)); break;
     case 2: DZ_CUDA_OK(launch_pdl(paged_decode_attention_kernel<T, 2>, grid, dim3(256), st, qkv, q_row_stride, out, kc, vc, bt, max_blocks, sl, block_size, kv_heads, scale, splits, partial, tickets)); break;
-    case 4: DZ_CUDA_OK(launch_pdl(paged_decode_attention_kernel<T, 4>, grid, dim3(256), st, qkv, q_row_stride, out, kc, vc, bt, max_blocks, sl, block_size, kv_heads, scale, splits, partial, tickets)); break;
-    case 8: DZ_CUDA_OK(launch_pdl(paged_decode_attention_kernel<T, 8>, grid, dim3(256), st, qkv, q_row_stride, out, kc, vc, bt, max_blocks, sl, block_size, kv_heads, scale, splits, partial, tickets)); break;
     default: return DZ_ERR_UNSUPPORTED;
   }
   return DZ_OK;
@@ -488,7 +420,7 @@ int dz_rotary_and_cache(void* qkv, const int64_t* positions, const int64_t* slot
 size_t dz_paged_attention_workspace_bytes(int num_seqs, int q_heads, int kv_heads, int splits) {
   if (num_seqs <= 0 || q_heads <= 0 || kv_heads <= 0 || splits <= 0) return 0;
   // tickets + partial triples
-  return kTicketBytes + (splits > 1 ? (size_t)num_seqs * q_heads * splits * (kHeadDim + 2) * 4 : 0);
+  return kTicketBytes + (splits > 1 ? grouped_decode_partial_bytes(num_seqs, q_heads, splits) : 0);
 }
 
 int dz_paged_attention_decode(const void* qkv, int q_row_stride, void* out, const void* k_cache,
@@ -518,6 +450,12 @@ int dz_paged_attention_decode(const void* qkv, int q_row_stride, void* out, cons
   cudaStream_t st = (cudaStream_t)stream;
   const dim3 grid(kv_heads, num_seqs, splits);
   const int group = q_heads / kv_heads;
+  if (group == 4 || group == 8) {
+    const GroupedDecode p = {qkv, q_row_stride, out, k_cache, v_cache, block_tables, max_blocks, block_size, seq_lens, 0,
+                             q_heads, kv_heads, scale, 0, nullptr, 0, nullptr, 1, splits,
+                             splits > 1 ? grouped_decode_partial(partial) : nullptr, tickets};
+    return launch_grouped_decode(p, num_seqs, dtype, st);
+  }
   if (dtype == DZ_DTYPE_F16)
     return attention_dispatch<__half>(group, grid, st, (const __half*)qkv, q_row_stride, (__half*)out,
                                       (const __half*)k_cache, (const __half*)v_cache, block_tables,

@@ -144,6 +144,8 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
   lo = Cvt<T>::down(a - h.x, b - h.y);
 }
 
+constexpr float kLog2e = 1.4426950408889634f;
+
 // -- launches --------------------------------------------------------------------------------------
 template <typename K, typename... Args>
 cudaError_t launch_ex(K kern, dim3 grid, dim3 block, size_t smem, int cluster_x, cudaStream_t st, Args... args) {

@@ -19,6 +19,7 @@
 //
 // Scores, softmax weights and sums are 32-bit.  In the tensor-core kernel a weight enters its
 // product with v as a hi + lo pair of 16-bit numbers.
+#include "dz_grouped_decode.cuh"
 #include "dz_window_attention.cuh"
 
 namespace dz {
@@ -640,6 +641,10 @@ int decode_group(int heads, int kv_heads) {
   const int r = heads / kv_heads;
   return r == 1 ? 1 : r == 2 ? 2 : 4;
 }
+// Query heads that share a key are rows of one MMA where the head sizes fit it.
+bool grouped_decode_fits(const AttnParams& p) {
+  return p.heads / p.kv_heads > 2 && p.dim == kGroupedDim && p.vdim == kGroupedDim;
+}
 int decode_grid_x(int heads, int kv_heads) {
   const int r = heads / kv_heads, g = decode_group(heads, kv_heads);
   return kv_heads * ((r + g - 1) / g);
@@ -698,7 +703,8 @@ int dz_kv_append(const void* qkv, int64_t row_stride, int k_off, int k_width, in
 size_t dz_window_attention_workspace_bytes(int num_seqs, int heads, int kv_heads, int vdim, int splits) {
   if (num_seqs <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || vdim <= 0) return 0;
   if (splits <= 1) return kAttnStatusBytes;
-  return kAttnStatusBytes + kTicketBytes + (size_t)num_seqs * heads * splits * (vdim + 2) * 4;
+  const size_t scratch = (size_t)num_seqs * heads * splits * (vdim + 2) * 4;
+  return kAttnStatusBytes + kTicketBytes + (vdim == kGroupedDim ? grouped_decode_partial_bytes(num_seqs, heads, splits) : scratch);
 }
 
 int dz_window_attention(const dz_window_attention_args* a, void* stream) {
@@ -734,6 +740,13 @@ int dz_window_attention(const dz_window_attention_args* a, void* stream) {
       tickets = (int*)((uint8_t*)a->workspace + kAttnStatusBytes);
       partial = (float*)((uint8_t*)tickets + kTicketBytes);
       if ((int64_t)a->num_seqs * decode_grid_x(a->heads, a->kv_heads) > kMaxTickets) return DZ_ERR_TOO_LARGE;
+    }
+    if (grouped_decode_fits(p)) {
+      const GroupedDecode d = {a->qkv, a->row_stride, a->out, a->k_cache, a->v_cache, a->block_tables, a->ring_blocks,
+                               a->block_size, a->ctx_lens, 1, a->heads, a->kv_heads, a->scale, max(a->window, 0), a->bias,
+                               a->bias_len, a->sink, 0, a->splits, a->splits > 1 ? grouped_decode_partial(partial) : nullptr,
+                               tickets};
+      return launch_grouped_decode(d, a->num_seqs, a->dtype, st);
     }
     const dim3 grid(decode_grid_x(a->heads, a->kv_heads), a->num_seqs, a->splits);
     const int g = decode_group(a->heads, a->kv_heads);

@@ -53,8 +53,6 @@ struct KeyRows {
   }
 };
 
-constexpr float kLog2e = 1.4426950408889634f;
-
 // dz_window_attention.cu: any type, any sizes, one CTA per (row, head)
 int launch_attention_any(const AttnParams& p, int num_seqs, int dtype, cudaStream_t st);
 

@@ -34,6 +34,8 @@ FUSED_MAX_TOKENS = 512
 # library GEMM, as the reference's PyTorch path does (deltazip/nn_modules/qlinear.py:266-330);
 # the SBMM kernel would expand the slot's codes once per 32-row window instead.
 DENSE_RUN_TOKENS = 256
+# Decode attention of grouped query heads: keys a CTA should have where the keys are split.
+GROUPED_MIN_KEYS = 128
 
 
 def _stream() -> int:
@@ -581,12 +583,21 @@ def rotary_and_cache(qkv: torch.Tensor, positions: torch.Tensor, q_heads: int, k
 _attn_ws = {}
 
 
+def _grouped_splits(seqs: int, heads: int, kv_heads: int, most_keys: int, at_least: int) -> int:
+    """Parts of every sequence's keys where several query heads share a key (the kernel on warp MMAs, two CTAs per SM):
+    `at_least` of them, and as many as one round of CTAs takes while each keeps GROUPED_MIN_KEYS.  A CTA costs about 5 us
+    beside its keys, so a second round never paid (160 sequences x 8 heads, 600 keys: 51 us in one part, 83 in two),
+    while a batch that leaves SMs idle gains until they are filled (1 x 8, 4000 keys: 52 us in one part, 20 in 16)."""
+    columns = seqs * kv_heads * -(-(heads // kv_heads) // 8)
+    return max(at_least, min(64, most_keys // GROUPED_MIN_KEYS, 296 // max(1, columns)))
+
+
 def paged_attention_decode(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                            block_tables: torch.Tensor, seq_lens: torch.Tensor, q_heads: int,
                            kv_heads: int, block_size: int, scale: float, splits: int = 1,
                            out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One query token per sequence (the q part of fused qkv rows [B, (q+2kv)*128]) against the
-    paged cache; returns [B, q_heads*128]."""
+    paged cache; returns [B, q_heads*128].  `splits`: CTAs that share a sequence's keys, at least."""
     _need_cuda(qkv, k_cache, v_cache, block_tables, seq_lens)
     b = qkv.shape[0]
     if block_tables.dtype != torch.int32 or seq_lens.dtype != torch.int32 or not block_tables.is_contiguous():
@@ -594,6 +605,8 @@ def paged_attention_decode(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: to
     if out is None:
         out = torch.empty((b, q_heads * 128), dtype=qkv.dtype, device=qkv.device)
     ws_ptr, ws_bytes = None, 0
+    if q_heads // kv_heads > 2:
+        splits = _grouped_splits(b, q_heads, kv_heads, block_tables.shape[1] * block_size, splits)
     if splits > 1:
         need = lib().dz_paged_attention_workspace_bytes(b, q_heads, kv_heads, splits)
         key = (qkv.device.index, _stream())
@@ -759,9 +772,12 @@ def window_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
         splits = 1
     elif splits <= 0:
         ratio = heads // kv_heads
-        ctas = seqs * kv_heads * ((ratio + 3) // 4 if ratio > 2 else 1)
-        most = (window + 63) // 64 if window > 0 else 8
-        splits = max(1, min(8, most, 296 // max(1, ctas)))
+        if ratio > 2 and dim == 128 and vdim == 128 and qkv.dtype != torch.float32:
+            splits = _grouped_splits(seqs, heads, kv_heads, block_tables.shape[1] * block_size, 1)
+        else:
+            ctas = seqs * kv_heads * ((ratio + 3) // 4 if ratio > 2 else 1)
+            most = (window + 63) // 64 if window > 0 else 8
+            splits = max(1, min(8, most, 296 // max(1, ctas)))
     ws = _zeroed_scratch("window_attention", qkv.device,
                          lib().dz_window_attention_workspace_bytes(seqs, heads, kv_heads, vdim, splits))
     args = _lib.WindowAttentionArgs(

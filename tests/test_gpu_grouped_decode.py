@@ -1,0 +1,86 @@
+"""Decode attention with several query heads per key/value head (warp MMAs) against softmax attention in 64 bits:
+lengths around its 16-key tiles, four warps and splits, group sizes that fill the eight MMA rows or not, windows,
+distance bias and sinks.
+
+Tolerance: scores and sums are 32-bit and a weight enters as two 16-bit parts, so what is left is the output's
+rounding, at most half a unit in the last place: 2^-11 (fp16) or 2^-8 (bf16) of every element; twice that for the
+relative 2-norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BLOCK = 16
+TOL = {torch.float16: 2 * 2.0 ** -11, torch.bfloat16: 2 * 2.0 ** -8}
+LENS = [1, 15, 16, 17, 63, 64, 65, 130, 257, 700]
+
+
+def batch(kvh, heads, dtype, seed, blocks_per_seq, lens):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(dtype)
+    n = len(lens)
+    tables = torch.randperm(n * blocks_per_seq, generator=g, device="cuda").to(torch.int32).view(n, blocks_per_seq)
+    rows = n * blocks_per_seq * BLOCK
+    return rnd(n, (heads + 2 * kvh) * 128), 2 * rnd(rows, kvh, 128), rnd(rows, kvh, 128), tables.contiguous()
+
+
+def reference(q, k, v, scale, bias=None, sink=None):
+    """q [heads, 128], k and v [keys, kv_heads, 128], bias [heads, keys], sink [heads]; 64 bits."""
+    rep = q.shape[0] // k.shape[1]
+    k, v = (t.double().repeat_interleave(rep, 1) for t in (k, v))
+    s = torch.einsum("hd,khd->hk", q.double(), k) * scale
+    if bias is not None:
+        s = s + bias.double()
+    if sink is not None:
+        s = torch.cat([s, sink.double()[:, None]], 1)
+    p = s.softmax(1)[:, :k.shape[0]]
+    return torch.einsum("hk,khd->hd", p, v).reshape(-1)
+
+
+def check(out, want, dtype):
+    assert torch.isfinite(out).all()
+    err = (out.double() - want).norm() / want.norm()
+    assert err <= TOL[dtype], float(err)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("heads,kvh", [(4, 1), (8, 1), (12, 3), (32, 4)])
+@pytest.mark.parametrize("splits", [1, 3, 33])
+def test_paged(heads, kvh, splits, dtype):
+    from deltazip_b200 import ops
+    qkv, k, v, tables = batch(kvh, heads, dtype, heads + splits, -(-max(LENS) // BLOCK), LENS)
+    lens = torch.tensor(LENS, dtype=torch.int32, device="cuda")
+    for rep in range(2):                           # twice: the tickets are back at zero
+        out = ops.paged_attention_decode(qkv, k, v, tables, lens, heads, kvh, BLOCK, 128 ** -0.5, splits)
+        for i, n in enumerate(LENS):
+            at = (tables[i].long()[:, None] * BLOCK + torch.arange(BLOCK, device="cuda")).flatten()[:n]
+            check(out[i], reference(qkv[i, :heads * 128].view(heads, 128), k[at], v[at], 128 ** -0.5), dtype)
+
+
+def test_paged_without_keys():
+    from deltazip_b200 import ops
+    qkv, k, v, tables = batch(1, 8, torch.float16, 1, 2, [0, 5])
+    out = ops.paged_attention_decode(qkv, k, v, tables, torch.tensor([0, 5], dtype=torch.int32, device="cuda"), 8, 1, BLOCK, 0.1)
+    assert not out[0].any() and out[1].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("heads,kvh", [(3, 1), (10, 2), (8, 1), (20, 2)])
+@pytest.mark.parametrize("window,splits,extra", [(300, 0, True), (300, 5, False), (33, 2, True), (5000, 0, True), (0, 3, False)])
+def test_window(heads, kvh, window, splits, extra, dtype):
+    from deltazip_b200 import ops
+    most = max(LENS) if window == 0 else min(window, max(LENS))
+    ring = -(-most // BLOCK)
+    qkv, k, v, tables = batch(kvh, heads, dtype, heads + window, ring, LENS)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    bias = torch.randn((heads, 40), generator=g, device="cuda") * 2 if extra else None
+    sink = torch.randn(heads, generator=g, device="cuda") if extra else None
+    starts = torch.arange(len(LENS) + 1, dtype=torch.int32, device="cuda")
+    ctx = torch.tensor([n - 1 for n in LENS], dtype=torch.int32, device="cuda")
+    for rep in range(2):
+        out = ops.window_attention(qkv, k, v, tables, starts, ctx, 1, True, heads, BLOCK, 0.11, window, bias, splits, sink)
+        for i, n in enumerate(LENS):
+            pos = torch.arange(max(0, n - window) if window else 0, n, device="cuda")
+            at = tables[i].long()[pos // BLOCK % ring] * BLOCK + pos % BLOCK
+            b = bias[:, (n - 1 - pos).clamp(max=39)] if extra else None
+            check(out[i], reference(qkv[i, :heads * 128].view(heads, 128), k[at], v[at], 0.11, b, sink), dtype)
