@@ -203,6 +203,15 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* v) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -290,6 +299,18 @@ __device__ __forceinline__ void warp_umma_ss(uint32_t d, uint32_t a_lo, uint32_t
       "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc)
       : "memory");
 }
+// One 2:4-sparse MMA (32 dense k): compressed A and metadata in tensor memory, B in shared memory.
+__device__ __forceinline__ void warp_umma_ts_sp(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t e_tmem, uint32_t idesc,
+                                                uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "@e tcgen05.mma.sp.cta_group::1.kind::f16 [%0], [%1], db, [%3], %5, p;\n\t}" ::"r"(d),
+      "r"(a), "r"(b_lo), "r"(e_tmem), "r"(kDescHi), "r"(idesc), "r"(acc)
+      : "memory");
+}
 __device__ __forceinline__ void warp_umma_commit(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
@@ -302,6 +323,13 @@ __device__ __forceinline__ void warp_tma_load_2d(uint32_t dst, const CUtensorMap
       "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(
           dst),
       "l"(map), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void warp_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void warp_mbar_expect_tx(uint32_t bar, uint32_t bytes) {
