@@ -9,8 +9,9 @@
 //
 // Two kernels.  The recurrent one streams the state once per token; it serves decoding, where its last
 // CTA of a sequence also does the norm and the gate, and the 32-bit type.  The chunkwise one takes 64
-// tokens at a time on the tensor cores for prompt portions.
-#include "dz_elem.cuh"
+// tokens at a time on the tensor cores for prompt portions; heads of 128 x 128 have one of their own
+// (dz_recurrent_tc.cu).
+#include "dz_recurrent_tc.cuh"
 
 namespace dz {
 namespace {
@@ -35,7 +36,6 @@ struct LightningParams {
 };
 
 __device__ __forceinline__ float silu_exact(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 
 // out = o / sqrt(mean(o^2) + eps) * w * sigmoid(g) over the n columns of one row, by one CTA
 template <typename T, typename I, int VEC>
@@ -220,16 +220,6 @@ __device__ __forceinline__ void bar_arrive(int id, int count) {
 
 template <int VT> __host__ __device__ constexpr int chunk_ldv() { return VT + 8; }
 template <int VT> __host__ __device__ inline int stage_elems(int dimp) { return kL * (2 * (dimp + 8) + 3 * chunk_ldv<VT>()); }
-
-template <typename T> __device__ __forceinline__ uint4 silu8(const uint4& v) {
-  uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = Cvt<T>::up(w[j]);
-    w[j] = Cvt<T>::down(silu_fast(f.x), silu_fast(f.y));
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
 
 template <typename T, int VT, int NTW>
 __global__ void __launch_bounds__(kChunkThreads, 1)
@@ -592,6 +582,16 @@ int dz_lightning(const dz_lightning_args* a, void* stream) {
   if (!dz_lightning_chunk_supported(a->dim, a->vdim, a->dtype)) return DZ_ERR_UNSUPPORTED;
   if (a->row_stride % 8 || a->k_off % 8 || a->v_off % 8 || !aligned16(a->x) || !aligned16(a->out)) return DZ_ERR_ALIGNMENT;
   int rc = DZ_OK;
+  if (a->dim == 128 && a->vdim == 128 && a->row_stride < (1ll << 31)) {
+    RecurrentParams r = {};
+    r.x = a->x; r.row_stride = a->row_stride; r.rows = a->rows; r.k_off = a->k_off; r.v_off = a->v_off;
+    r.out = a->out; r.S = a->S; r.slots = a->slots; r.q_starts = a->q_starts; r.ctx_lens = a->ctx_lens;
+    r.heads = a->heads; r.powers = a->powers;
+    r.status = recurrent_status(a->workspace, a->workspace_bytes, 0);
+    rc = launch_recurrent_tc(r, false, a->dtype, a->num_seqs, st);
+    if (rc) return rc;
+    DZ_DISPATCH16(a->dtype, return (run_norm<T, T>(p, (const T*)p.out, a->rows, st)));
+  }
   DZ_DISPATCH16(a->dtype, rc = run_chunk<T>(p, a->num_seqs, (a->dim + 15) / 16 * 16, st));
   if (rc) return rc;
   DZ_DISPATCH16(a->dtype, return (run_norm<T, T>(p, (const T*)p.out, a->rows, st)));

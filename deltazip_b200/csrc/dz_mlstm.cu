@@ -10,10 +10,11 @@
 //
 // Two kernels.  The recurrent one streams the state once per token and also does what follows the
 // cell (per-head RMS norm, weight, sigmoid output gate); it serves decoding and the 32-bit type.  The
-// chunkwise one takes 64 tokens at a time on the tensor cores for prompt portions.
+// chunkwise one takes 64 tokens at a time on the tensor cores for prompt portions; heads of 128 x 128
+// have one of their own (dz_recurrent_tc.cu).
 #include <cooperative_groups.h>
 
-#include "dz_elem.cuh"
+#include "dz_recurrent_tc.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -41,9 +42,6 @@ struct MlstmParams {
   const int* ctx_lens;
   int heads, dim, vdim;
 };
-
-__device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ float soft_cap(float x, float cap) { return cap * tanhf(x / cap); }
 
 // -------------------------------------------------------------------------------------------------
 // Recurrent form.  A cluster of C CTAs owns one (head, sequence); CTA r holds columns
@@ -672,6 +670,15 @@ int dz_mlstm(const dz_mlstm_args* a, void* stream) {
   if (a->row_stride % 8 || a->k_off % 8 || a->v_off % 8 || a->g_off % 8 || !aligned16(a->x) || !aligned16(a->out))
     return DZ_ERR_ALIGNMENT;
   if (!a->workspace || a->workspace_bytes < dz_mlstm_workspace_bytes(a->num_seqs, a->heads)) return DZ_ERR_WORKSPACE;
+  if (a->dim == 128 && a->vdim == 128 && a->row_stride < (1ll << 31)) {
+    RecurrentParams r = {};
+    r.x = a->x; r.row_stride = a->row_stride; r.rows = a->rows; r.k_off = a->k_off; r.v_off = a->v_off; r.g_off = a->g_off;
+    r.out = a->out; r.S = a->S; r.slots = a->slots; r.q_starts = a->q_starts; r.ctx_lens = a->ctx_lens;
+    r.heads = a->heads; r.pre_if = a->pre_if; r.b_if = a->b_if; r.cap = a->cap; r.scale = a->scale;
+    r.n = a->n; r.m = a->m; r.norm_w = a->norm_weight; r.eps = a->eps;
+    r.status = recurrent_status(a->workspace, a->workspace_bytes, dz_mlstm_workspace_bytes(a->num_seqs, a->heads));
+    return launch_recurrent_tc(r, true, a->dtype, a->num_seqs, st);
+  }
   const int dimp = (a->dim + 15) / 16 * 16;
   int rc = DZ_OK;
   const bool wide = a->vdim > 32 && dimp <= 256 && chunk_smem(dimp, 64) <= kMaxDynSmem;

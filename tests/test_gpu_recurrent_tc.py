@@ -1,0 +1,71 @@
+"""Chunkwise recurrences with heads of 128 x 128 (the tcgen05 kernel): chunk borders, continued sequences, decays and
+gates at their ends, unequal batches -- against the 64-bit recurrences of the oracle."""
+import pytest
+import torch
+
+from tests.test_gpu_buzalorn import BF16, EXACT, F16, MlstmRun, i32, rel
+from tests.test_gpu_movarax import LightningRun
+
+pytestmark = pytest.mark.gpu
+
+# whole chunks, one token more and less, single tokens between portions; then prompts continued from decoding
+CUTS = [[600], [127, 1, 128, 129, 215], [256, 256, 88], [5, 300], [1, 130]]
+CHUNKS = lambda n: n > 4
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16])
+@pytest.mark.parametrize("run", [MlstmRun, LightningRun])
+def test_chunk_borders(run, dtype):
+    r = run(2, 128, 128, 600, dtype)
+    for cuts in CUTS:
+        always = len(cuts) != 2
+        assert rel(r.run(cuts, chunk=lambda n: always or n > 4), r.want) < EXACT[dtype], cuts
+    assert torch.isnan(r.S[0]).all() and torch.isnan(r.S[2]).all()
+
+
+@pytest.mark.parametrize("kw", [dict(f_mean=-30.0, cap=12.0), dict(f_mean=30.0, cap=14.0), dict(i_std=40.0, cap=13.0)])
+def test_gates_at_their_ends(kw):
+    r = MlstmRun(2, 128, 128, 300, BF16, seed=5, **kw)
+    for cuts in ([300], [130, 40]):
+        assert rel(r.run(cuts, chunk=CHUNKS), r.want) < EXACT[BF16] * 1.5, cuts
+
+
+def test_decays_at_their_ends():
+    r = LightningRun(3, 128, 128, 400, BF16, decay=[0.0, 1.0, 0.999])
+    for cuts in ([400], [129, 131]):
+        assert rel(r.run(cuts, chunk=CHUNKS), r.want) < EXACT[BF16], cuts
+
+
+def test_absent_tokens_bring_nothing_from_their_neighbours():
+    """Rows behind a sequence's end hold infinities: they belong to the next one."""
+    from deltazip_b200 import ops
+    a = LightningRun(2, 128, 128, 131, BF16, seed=3)
+    x = torch.cat([a.x, torch.full_like(a.x[:100], float("inf"))])
+    S = torch.zeros(3, 2, 128, 128, device="cuda")
+    got = ops.lightning(x, a.powers, a.norm, S, i32([1, 2]), i32([0, 131, 231]), i32([0, 0]), a.eps, True)
+    assert rel(got[:131].double().cpu().numpy(), a.want) < EXACT[BF16] and torch.isfinite(S[1]).all()
+    b = MlstmRun(2, 128, 128, 131, BF16, seed=3)
+    x = torch.cat([b.x, torch.full_like(b.x[:100], float("inf"))])
+    h = torch.cat([b.h, b.h[:100]])
+    S, n, m = torch.zeros(3, 2, 128, 128, device="cuda"), torch.zeros(3, 2, 128, device="cuda"), torch.zeros(3, 2, device="cuda")
+    got = ops.mlstm(x, h, b.w, b.b, b.norm, S, n, m, i32([1, 2]), i32([0, 131, 231]), i32([0, 0]), b.cap, b.scale, b.eps, True)
+    assert rel(got[:131].double().cpu().numpy(), b.want) < EXACT[BF16] and torch.isfinite(S[1]).all()
+
+
+def test_unequal_sequences_in_one_batch():
+    from deltazip_b200 import ops
+    runs = [MlstmRun(2, 128, 128, t, BF16, seed=t) for t in (290, 3, 128)]
+    w, b, norm = runs[0].w, runs[0].b, runs[0].norm
+    S, n, m = torch.zeros(5, 2, 128, 128, device="cuda"), torch.zeros(5, 2, 128, device="cuda"), torch.zeros(5, 2, device="cuda")
+    x, h = torch.cat([r.x for r in runs]), torch.cat([r.h for r in runs])
+    args = (runs[0].cap, runs[0].scale, runs[0].eps)
+    got = ops.mlstm(x, h, w, b, norm, S, n, m, i32([3, 0, 4, 2]), i32([0, 290, 293, 293, 421]), i32([0, 0, 0, 0]), *args, True)
+    at = 0
+    for r, slot in zip(runs, (3, 0, 2)):
+        s1, n1, m1 = torch.zeros_like(S), torch.zeros_like(n), torch.zeros_like(m)
+        alone = ops.mlstm(r.x, r.h, w, b, norm, s1, n1, m1, i32([1]), i32([0, r.t]), i32([0]), *args, True)
+        assert torch.equal(alone, got[at:at + r.t]) and torch.equal(s1[1], S[slot]) and torch.equal(n1[1], n[slot])
+        assert torch.equal(m1[1], m[slot])
+        at += r.t
+    assert not S[4].any() and not m[4].any()              # no tokens: the slot is left alone
+    assert ops.read_status(x.device) == 0
