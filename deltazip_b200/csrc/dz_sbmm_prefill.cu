@@ -7,19 +7,18 @@
 // instead of once per 32-token window, and B is the x tile as TMA brings it -- columns past the end of the run are
 // computed and not stored, so no row has to be masked or copied.
 //
-// With F = 2 an x tile serves 256 features: x is what a unit moves most of (45 KB of x to 6 KB of codes), and it
-// comes out of L2 at about 40 bytes per cycle and SM.  F = 1 makes twice as many tiles, which layers of few
-// features need to fill the SMs evenly.
+// With F = 2 an x tile serves 256 features: x is what a unit moves most of (45 KB of x to 6 KB of codes).  F = 1 is for
+// an odd number of feature groups.
 //
-// Measured on the four projections of a 7B decoder layer, 1999 tokens in seven runs, 4-bit: 4560 -> 1457 us with the
+// Measured on the four projections of a 7B decoder layer, 1999 tokens in seven runs, 4-bit: 4700 -> 1281 us with the
 // dense products (about 550 of them), against one pass of the decode kernel per 128 tokens.
 //
-// Roles: a TMA producer (x), a bulk-copy producer (packed stages), an MMA issuer, two warpgroups that expand, two
+// Roles: a TMA producer (x), a bulk-copy producer (packed stages), F MMA issuers, two warpgroups that expand, two
 // that drain one accumulator each and add it to y.  All waits are bounded.
 #include <cuda.h>
-#include <cuda_bf16.h>
+#include <type_traits>
 
-#include "dz_common.cuh"
+#include "dz_elem.cuh"
 #include "dz_expand.cuh"
 #include "dz_tc.cuh"
 
@@ -29,7 +28,7 @@ namespace {
 constexpr int kPTokens = 176;                  // most columns of a token block
 constexpr int kPBoxRows = 88;                  // rows of one TMA copy of x (one or two per half-tile)
 constexpr int kPThreads = 20 * 32;             // 4 service warps, 2 x 4 expanding, 2 x 4 draining
-constexpr int kPXStages = 6, kPXBytes = kPTokens * 128;       // half-tiles of 64 k
+constexpr int kPXHalf = kPTokens * 128, kPXStages = 3, kPXBytes = 2 * kPXHalf;    // a unit's two half-tiles of 64 k
 constexpr int kPRStages = 8;
 constexpr int kPTmemCols = 512;
 // tensor memory: two accumulators, four buffers of expanded A (32 columns) and of metadata (4)
@@ -81,20 +80,22 @@ __device__ __forceinline__ PTile tile_at(int v, const PParams& p, const int* fir
 template <int BITS, int DT>
 __global__ void __launch_bounds__(kPThreads, 1)
 sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) {
+  using T = typename std::conditional<DT == 0, __half, __nv_bfloat16>::type;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t s_xfull[kPXStages], s_xempty[kPXStages], s_rfull[kPRStages], s_rempty[kPRStages],
       s_aready[4], s_afree[4], s_accfull[2], s_accempty[2];
   __shared__ int s_begin[kPrefillMaxSlots], s_end[kPrefillMaxSlots], s_first[kPrefillMaxSlots + 1];
+  __shared__ int s_tok[2][kPTokens];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t s_x = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t s_r = s_x + kPXStages * kPXBytes;
   volatile int* abort_flag = &s_abort;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kPXStages; ++i) { mbar_init(smem_u32(&s_xfull[i]), 1); mbar_init(smem_u32(&s_xempty[i]), 1); }
+    for (int i = 0; i < kPXStages; ++i) { mbar_init(smem_u32(&s_xfull[i]), 1); mbar_init(smem_u32(&s_xempty[i]), p.F); }
     for (int i = 0; i < kPRStages; ++i) { mbar_init(smem_u32(&s_rfull[i]), 1); mbar_init(smem_u32(&s_rempty[i]), 128); }
     for (int i = 0; i < 4; ++i) { mbar_init(smem_u32(&s_aready[i]), 128); mbar_init(smem_u32(&s_afree[i]), 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&s_accfull[i]), 1); mbar_init(smem_u32(&s_accempty[i]), 128); }
@@ -149,18 +150,21 @@ sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) 
   const int F = p.F;
 
   if (warp == 0) {
-    // ---- x half-tiles ----
+    // ---- x ----
     Ring rx(kPXStages, 1);
     for (int v = blockIdx.x; v < total; v += gridDim.x) {
       const PTile t = tile_at(v, p, s_first, s_begin, s_end);
-      const bool two = t.rows > kPBoxRows;
-      for (int kb = 0; kb < p.num_kblocks; ++kb) {
+      const int boxes = t.rows > kPBoxRows ? 2 : 1;
+      for (int ku = 0; ku < p.num_kunits; ++ku) {
+        const int nhalf = min(2, p.num_kblocks - ku * 2);
         bar_wait(&s_xempty[rx.idx], rx.par, abort_flag, p.status);
         __syncwarp();
-        const uint32_t full = smem_u32(&s_xfull[rx.idx]), dst = s_x + rx.idx * kPXBytes;
-        warp_mbar_expect_tx(full, (two ? 2 : 1) * kPBoxRows * 128);
-        warp_tma_load_2d(dst, &map_x, kb * kBlockK, t.row0, full);
-        if (two) warp_tma_load_2d(dst + kPBoxRows * 128, &map_x, kb * kBlockK, t.row0 + kPBoxRows, full);
+        const uint32_t full = smem_u32(&s_xfull[rx.idx]);
+        warp_mbar_expect_tx(full, nhalf * boxes * kPBoxRows * 128);
+        for (int h = 0; h < nhalf; ++h)
+          for (int b = 0; b < boxes; ++b)
+            warp_tma_load_2d(s_x + rx.idx * kPXBytes + h * kPXHalf + b * (kPBoxRows * 128), &map_x, (ku * 2 + h) * kBlockK,
+                             t.row0 + b * kPBoxRows, full);
         rx.advance();
       }
     }
@@ -185,51 +189,42 @@ sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) 
         }
       }
     }
-  } else if (warp == 1) {
-    // ---- MMA issuer ----
+  } else if (warp == 1 || (warp == 3 && F == 2)) {
+    // ---- MMA issue: with two feature groups a warp for each (one warp takes 900 cycles to a unit of two groups,
+    // waits and commits included, and the MMAs of 176 columns 700; their accumulators are independent) ----
+    const int mine = F == 2 ? warp >> 1 : 0;
     Ring rx(kPXStages, 0);
-    int stage = 0, tiles = 0;
-    for (int v = blockIdx.x; v < total; v += gridDim.x) {
+    int stage = mine, tiles = 0;
+    const int whole = p.num_kblocks / 2;
+    for (int v = blockIdx.x; v < total; v += gridDim.x, ++tiles) {
       const PTile t = tile_at(v, p, s_first, s_begin, s_end);
       const uint32_t idesc = make_idesc<DT>((t.rows + 15) & ~15, true);
       // F = 2: group f in accumulator f; F = 1: tiles alternate between the accumulators
-      for (int f = 0; f < F; ++f) {
-        const int d = F == 2 ? f : tiles & 1, use = F == 2 ? tiles : tiles >> 1;
-        bar_wait(&s_accempty[d], (use & 1) ^ 1, abort_flag, p.status);
-      }
-      __syncwarp();
-      tc_fence_after();
-      for (int ku = 0; ku < p.num_kunits; ++ku) {
-        const int nhalf = min(2, p.num_kblocks - ku * 2);
-        const int x0 = rx.idx;
+      const int acc = F == 2 ? mine : tiles & 1, use = F == 2 ? tiles : tiles >> 1;
+      const uint32_t d = tmem + acc * kPAcc1;
+      bar_wait(&s_accempty[acc], (use & 1) ^ 1, abort_flag, p.status);
+      for (int ku = 0; ku < p.num_kunits; ++ku, stage += F) {
+        const int buf = (stage & 1) + 2 * ((stage >> 1) & 1);
         bar_wait(&s_xfull[rx.idx], rx.par, abort_flag, p.status);
-        rx.advance();
-        const int x1 = rx.idx;
-        if (nhalf == 2) {
-          bar_wait(&s_xfull[rx.idx], rx.par, abort_flag, p.status);
-          rx.advance();
-        }
-        for (int f = 0; f < F; ++f, ++stage) {
-          const int buf = (stage & 1) + 2 * ((stage >> 1) & 1);
-          bar_wait(&s_aready[buf], (stage >> 2) & 1, abort_flag, p.status);
-          __syncwarp();
-          tc_fence_after();
-          const uint32_t d = tmem + (F == 2 ? f : tiles & 1) * kPAcc1;
-          const uint32_t a = tmem + kPACol + buf * 32, e = tmem + kPECol + buf * 4;
-          const uint32_t b0 = desc_lo(s_x + x0 * kPXBytes), b1 = desc_lo(s_x + x1 * kPXBytes);
+        bar_wait(&s_aready[buf], (stage >> 2) & 1, abort_flag, p.status);
+        __syncwarp();
+        tc_fence_after();
+        const uint32_t b0 = desc_lo(s_x + rx.idx * kPXBytes), b1 = b0 + (kPXHalf >> 4);
+        const uint32_t a = tmem + kPACol + buf * 32, e = tmem + kPECol + buf * 4;
+        if (ku < whole) {                                // (a branch between the MMAs would cost them their uniform registers)
           warp_umma_ts_sp(d, a, b0, e, idesc, ku > 0);
           warp_umma_ts_sp(d, a + 8, b0 + 4, e, idesc | 1, 1);
-          if (nhalf == 2) {
-            warp_umma_ts_sp(d, a + 16, b1, e + 2, idesc, 1);
-            warp_umma_ts_sp(d, a + 24, b1 + 4, e + 2, idesc | 1, 1);
-          }
-          warp_umma_commit(smem_u32(&s_afree[buf]));
+          warp_umma_ts_sp(d, a + 16, b1, e + 2, idesc, 1);
+          warp_umma_ts_sp(d, a + 24, b1 + 4, e + 2, idesc | 1, 1);
+        } else {                                         // K ends with half a unit
+          warp_umma_ts_sp(d, a, b0, e, idesc, ku > 0);
+          warp_umma_ts_sp(d, a + 8, b0 + 4, e, idesc | 1, 1);
         }
-        warp_umma_commit(smem_u32(&s_xempty[x0]));
-        if (nhalf == 2) warp_umma_commit(smem_u32(&s_xempty[x1]));
+        warp_umma_commit(smem_u32(&s_afree[buf]));
+        warp_umma_commit(smem_u32(&s_xempty[rx.idx]));
+        rx.advance();
       }
-      for (int f = 0; f < F; ++f) warp_umma_commit(smem_u32(&s_accfull[F == 2 ? f : tiles & 1]));
-      ++tiles;
+      warp_umma_commit(smem_u32(&s_accfull[acc]));
     }
   } else if (warp >= 4 && warp < 12) {
     // ---- expansion: warpgroup w takes the stages of its parity ----
@@ -244,8 +239,8 @@ sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) 
         const int ku = F == 2 ? i >> 1 : i;
         const bool both = ku * 2 + 1 < p.num_kblocks;
         const int s = stage + i, ri = s % kPRStages, buf = w + 2 * (n & 1);
-        mbar_wait(smem_u32(&s_rfull[ri]), (s / kPRStages) & 1, abort_flag, p.status);
-        mbar_wait(smem_u32(&s_afree[buf]), ((n >> 1) & 1) ^ 1, abort_flag, p.status);
+        bar_wait(&s_rfull[ri], (s / kPRStages) & 1, abort_flag, p.status);
+        bar_wait(&s_afree[buf], ((n >> 1) & 1) ^ 1, abort_flag, p.status);
         __syncwarp();
         tc_fence_after();
         const uint32_t raw = s_r + ri * p_stage_bytes(BITS);
@@ -281,7 +276,11 @@ sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) 
     // ---- warpgroup d drains accumulator d into y ----
     const int d = (warp - 12) >> 2, q = warp & 3, r = q * 32 + lane;
     const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + d * kPAcc1;
-    unsigned short* const y = reinterpret_cast<unsigned short*>(p.y);
+    auto drain_sync = [&]() {                            // this warpgroup
+      if (d == 0) named_bar_sync(1, 128);
+      else named_bar_sync(2, 128);
+    };
+    T* const y = reinterpret_cast<T*>(p.y);
     int tiles = 0, uses = 0;
     for (int v = blockIdx.x; v < total; v += gridDim.x) {
       const PTile t = tile_at(v, p, s_first, s_begin, s_end);
@@ -290,41 +289,55 @@ sbmm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const PParams p) 
       if (!mine) continue;
       const int n = (t.group0 + (F == 2 ? d : 0)) * kTileN + r;
       const float sc = __half2float(*reinterpret_cast<const __half*>(p.scales + (size_t)t.slot * p.sstride + (size_t)n * 2));
-      // y of 16 tokens at a time is requested one chunk ahead, the first before the wait
-      unsigned short old[16];
-      auto fetch = [&](int c) {
+      // A lane works on two features of every second token (its own sums and its neighbour's), so that y moves 32 bits
+      // at a time; 64 tokens of it are on their way before the sums are complete and from there on.
+      constexpr int kAhead = 4;
+      const int odd = lane & 1;
+      int* const tok = s_tok[d];
+      drain_sync();                        // the tile before has been read
+      for (int i = r; i < t.rows; i += 128) tok[i] = perm[t.row0 + i];
+      drain_sync();
+      uint32_t old[kAhead][8];
+      auto fetch = [&](uint32_t (&o)[8], int c) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c + i < t.rows) old[i] = y[(size_t)perm[t.row0 + c + i] * p.ldy + n];
+        for (int i = 0; i < 8; ++i) {
+          const int at = c + 2 * i + odd;
+          o[i] = at < t.rows ? *reinterpret_cast<const uint32_t*>(y + (size_t)tok[at] * p.ldy + (n - odd)) : 0;
+        }
       };
-      fetch(0);
-      mbar_wait(smem_u32(&s_accfull[d]), uses & 1, abort_flag, p.status);
+#pragma unroll
+      for (int g = 0; g < kAhead; ++g) fetch(old[g], g * 16);
+      bar_wait(&s_accfull[d], uses & 1, abort_flag, p.status);
       ++uses;
       __syncwarp();
       tc_fence_after();
-      for (int c = 0; c < t.rows; c += 16) {
-        uint32_t u[16];
-        tmem_ld16(acc + c, u);
-        tmem_wait_ld();
-        unsigned short now[16];
+      for (int c0 = 0; c0 < t.rows; c0 += 16 * kAhead) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) now[i] = old[i];
-        if (c + 16 < t.rows) {
-          fetch(c + 16);
-        } else {
-          tc_fence_before();
-          mbar_arrive(smem_u32(&s_accempty[d]));
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c + i < t.rows) {
-            const size_t at = (size_t)perm[t.row0 + c + i] * p.ldy + n;
-            if (DT == 0)
-              y[at] = __half_as_ushort(__float2half_rn(fmaf(sc, __uint_as_float(u[i]), __half2float(__ushort_as_half(now[i])))));
-            else
-              y[at] = __bfloat16_as_ushort(
-                  __float2bfloat16_rn(fmaf(sc, __uint_as_float(u[i]), __bfloat162float(__ushort_as_bfloat16(now[i])))));
+        for (int g = 0; g < kAhead; ++g) {
+          const int c = c0 + g * 16;
+          if (c >= t.rows) break;
+          uint32_t u[16];
+          tmem_ld16(acc + c, u);
+          tmem_wait_ld();
+          if (c + 16 >= t.rows) {
+            tc_fence_before();
+            mbar_arrive(smem_u32(&s_accempty[d]));
           }
+          uint32_t now[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float a = sc * __uint_as_float(u[2 * i]), b = sc * __uint_as_float(u[2 * i + 1]);
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            const float2 before = Cvt<T>::up(old[g][i]);
+            now[i] = odd ? Cvt<T>::down(before.x + got, before.y + b) : Cvt<T>::down(before.x + a, before.y + got);
+          }
+          fetch(old[g], c + 16 * kAhead);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int at = c + 2 * i + odd;
+            if (at < t.rows) *reinterpret_cast<uint32_t*>(y + (size_t)tok[at] * p.ldy + (n - odd)) = now[i];
+          }
+        }
       }
     }
   }
@@ -356,10 +369,9 @@ int launch_sbmm_prefill(const dz_sbmm_args& a, const void* xsrc, int sms, cudaSt
   p.num_kblocks = a.K / kBlockK;
   p.num_kunits = (p.num_kblocks + 1) / 2;
   p.groups = a.N / kTileN;
-  // Two feature groups a tile where that still leaves about four tiles for every SM (the last wave then
-  // costs less than the second pass over x).
-  const long long blocks = a.M / kPTokens + 1;
-  p.F = (p.groups % 2 == 0 && blocks * (p.groups / 2) >= 4ll * sms) ? 2 : 1;
+  // One feature group only where their number is odd: with two an x tile serves both and two warps issue (12288 x 4096,
+  // 2048 tokens: 125 us, with one 148; 4096 x 4096, whose 192 tiles fill 1.3 waves: 68 and 70).
+  p.F = p.groups % 2 == 0 ? 2 : 1;
   p.ldy = a.y_stride ? a.y_stride : a.N;
   p.qweight = (const uint8_t*)a.qweight; p.meta = (const uint8_t*)a.meta; p.scales = (const uint8_t*)a.scales;
   p.qstride = a.qweight_stride; p.mstride = a.meta_stride; p.sstride = a.scales_stride;
