@@ -6,10 +6,15 @@
 // are four products per chunk, 56 MMAs of 128 x 128 x 16.  The state, P and w V, held in 32 bits, enter them as hi +
 // lo pairs of the 16-bit type; the state itself stays in 32 bits in registers.
 //
+// Bound by the sixteen warps: of 10 to 13 thousand cycles a chunk SiLU takes 5 (lightning; the special function unit),
+// the exponentials and sums of the gates 4 and the output gate 5 (matrix memory), the products wait for them.
+// Measured against the warp-MMA kernels of 64 tokens at a time, bf16: matrix memory, 4 prompts of up to 2048 tokens x
+// 32 heads, 566 -> 170 us; constant decay, 5 prompts of up to 1500 x 16 heads, continued, 260 -> 133 us.
+//
 // Tensor memory (128 columns each): scores, then P in their place | O | the update | w V.
 // Shared memory: a ring of four tiles of 128 x 128 (q, k, v, q, ...) and S as the product with q reads it.
 // Roles: 16 warps work on what lies between the products -- a thread owns a row (lane) and 32 of its columns --, two
-// or three bring tiles in, one issues the MMAs, one computes the gates' weights a chunk ahead.  While a step of the 16
+// bring tiles in, one issues the MMAs, one computes the gates' weights a chunk ahead.  While a step of the 16
 // runs, the tensor cores do another product: scores and Q S under w V, the update under P, P V under the state's
 // update.  All waits are bounded.
 #include <cuda.h>
@@ -28,7 +33,7 @@ constexpr int kSlots = 4;
 // Twenty warps, the most that leave a thread 96 registers (32 of a worker's hold the state): the workers, one that
 // issues, with gates one that computes the weights, the rest bring tiles in.
 constexpr int kWorkWarps = 16, kIssueWarp = 19, kThreadsRec = 20 * 32;
-template <bool MEMORY> constexpr int kLoaders = MEMORY ? 64 : 96;
+constexpr int kLoaders = 64;
 constexpr int kTQk = 0, kTO = 128, kTU = 256, kTW = 384;     // columns of tensor memory
 constexpr float kDenEps = 1e-6f;
 constexpr size_t kSmemRec = (kSlots + 2) * kTileBytes + 1024;
@@ -69,10 +74,10 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
                                                                             const RecurrentParams p) {
   constexpr int DT = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
   extern __shared__ uint8_t smem_dyn[];
-  __shared__ __align__(8) uint64_t b_full[kSlots], b_raw[kSlots], b_empty[kSlots], b_wfull[2], b_wempty[2], b_qk, b_inter, b_u, b_pv, b_w,
+  __shared__ __align__(8) uint64_t b_full[kSlots], b_empty[kSlots], b_wfull[2], b_wempty[2], b_qk, b_inter, b_u, b_pv, b_k, b_w,
       b_p, b_s, b_ofree;
   __shared__ ChunkWeights s_cw[2];
-  __shared__ __align__(16) float s_n[kDim];
+  __shared__ __align__(16) float s_n[kDim], s_nw[kDim];
   __shared__ float s_np[4][kDim], s_nq[4][kTok], s_den[4][kTok], s_sq[4][kTok];
   __shared__ float s_pw[2 * kTok + 1];                   // w^i at [128 + i], zero before it
   __shared__ uint32_t s_tmem;
@@ -91,8 +96,7 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
 
   if (tid == 0) {
     for (int i = 0; i < kSlots; ++i) {
-      mbar_init(smem_u32(&b_full[i]), kLoaders<MEMORY>);
-      mbar_init(smem_u32(&b_raw[i]), 1);
+      mbar_init(smem_u32(&b_full[i]), kLoaders);
       mbar_init(smem_u32(&b_empty[i]), 1 + kWorkWarps);
     }
     for (int i = 0; i < 2; ++i) {
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       mbar_init(smem_u32(&b_wempty[i]), kWorkWarps);
     }
     for (uint64_t* b : {&b_qk, &b_inter, &b_u, &b_pv}) mbar_init(smem_u32(b), 1);
-    for (uint64_t* b : {&b_w, &b_p, &b_s, &b_ofree}) mbar_init(smem_u32(b), kWorkWarps);
+    for (uint64_t* b : {&b_k, &b_w, &b_p, &b_s, &b_ofree}) mbar_init(smem_u32(b), kWorkWarps);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
@@ -112,6 +116,7 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if constexpr (MEMORY) {
+    if (tid < kDim) s_nw[tid] = p.norm_w[(size_t)head * kDim + tid];
     if (tid < kDim) s_n[tid] = ctx > 0 ? p.n[((size_t)slot * p.heads + head) * kDim + tid] : 0.f;
   } else {
     for (int j = tid; j <= 2 * kTok; j += kThreadsRec) { // past the table: w^64 w^(i - 64)
@@ -160,15 +165,18 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       if constexpr (MEMORY) bar_wait(&b_wfull[i & 1], (i >> 1) & 1, abort_flag, p.status);
       bar_wait(&b_full[nv & 3], (nv >> 2) & 1, abort_flag, p.status);     // q and k came before it
       __syncwarp();
-      if constexpr (!MEMORY) {                           // q and k come through SiLU, v gets it here
-        const uint32_t at = s_ring + (nv & 3) * kTileBytes;
+      if constexpr (!MEMORY) {                           // q, k and v go through SiLU in place
+        for (int n = nq; n <= nv; ++n) {
+          const uint32_t at = s_ring + (n & 3) * kTileBytes;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int e = tid + j * kWorkWarps * 32;
-          const uint32_t a = at + swizzled(e >> 4, e & 15, kSlab);
-          sts128(a, silu8<T>(lds128(a)));
+          for (int j = 0; j < 4; ++j) {
+            const int e = tid + j * kWorkWarps * 32;
+            const uint32_t a = at + swizzled(e >> 4, e & 15, kSlab);
+            sts128(a, silu8<T>(lds128(a)));
+          }
+          fence_proxy_async();
+          if (n == nk) signal(&b_k);
         }
-        fence_proxy_async();
         named_bar_sync(1, kWorkWarps * 32);
       }
       // w V, transposed: this row's column of v
@@ -196,9 +204,14 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       if constexpr (MEMORY) {
         const uint32_t k_at = s_ring + (nk & 3) * kTileBytes + col;
         float sum = 0.f;
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j)
-          sum = fmaf(cw.w[c0 + j], lds_one<T>(k_at + (c0 + j) * 128 + ((col_chunk ^ (uint32_t)(j & 7)) << 4)), sum);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(cw.w + c0 + j);
+          const float wj[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            sum = fmaf(wj[e], lds_one<T>(k_at + (c0 + j + e) * 128 + ((col_chunk ^ (uint32_t)((j + e) & 7)) << 4)), sum);
+        }
         s_np[h][r] = sum;
         const uint32_t q_at = s_ring + (nq & 3) * kTileBytes;
         float dot = 0.f;
@@ -300,7 +313,11 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       const bool row_ok = r < len;
       T* op = (T*)p.out + (size_t)(q0 + base + (row_ok ? r : 0)) * p.heads * kDim + (size_t)head * kDim + c0;
       float inv = 1.f;
+      uint4 gate[MEMORY ? 4 : 1];
       if constexpr (MEMORY) {
+        const T* gp = (const T*)p.x + (size_t)(q0 + base + (row_ok ? r : 0)) * p.row_stride + p.g_off + (size_t)head * kDim + c0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) gate[c] = reinterpret_cast<const uint4*>(gp)[c];
         named_bar_sync(1, kWorkWarps * 32);              // everyone's parts of n, q.n and the sums of P
         float nq_sum = 0.f, ds = 0.f;
 #pragma unroll
@@ -318,7 +335,6 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       tc_fence_before();
       signal(&b_ofree);
       if constexpr (MEMORY) {
-        const T* gp = (const T*)p.x + (size_t)(q0 + base + (row_ok ? r : 0)) * p.row_stride + p.g_off + (size_t)head * kDim + c0;
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -329,13 +345,17 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
         named_bar_sync(1, kWorkWarps * 32);
         const float rms = 1.f / sqrtf(((s_sq[0][r] + s_sq[1][r]) + (s_sq[2][r] + s_sq[3][r])) / (float)kDim + p.eps);
         if (row_ok) {
-          const float* wp = p.norm_w + (size_t)head * kDim + c0;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            float e[8], f[8];
-            load8<T>(gp + c * 8, e);
+            const uint32_t g[4] = {gate[c].x, gate[c].y, gate[c].z, gate[c].w};
+            float f[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = o[c * 8 + j] * rms * wp[c * 8 + j] / (1.f + __expf(-e[j]));
+            for (int j = 0; j < 4; ++j) {
+              const float2 e = Cvt<T>::up(g[j]);
+              const int k = c * 8 + 2 * j;
+              f[2 * j] = __fdividef(o[k] * rms * s_nw[c0 + k], 1.f + __expf(-e.x));
+              f[2 * j + 1] = __fdividef(o[k + 1] * rms * s_nw[c0 + k + 1], 1.f + __expf(-e.y));
+            }
             store8<T>(op + c * 8, f);
           }
         }
@@ -354,52 +374,33 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
     if constexpr (MEMORY) {
       if (h == 0) p.n[((size_t)slot * p.heads + head) * kDim + r] = s_n[r];
     }
-  } else if (warp < kWorkWarps + kLoaders<MEMORY> / 32) {
+  } else if (warp < kWorkWarps + kLoaders / 32) {
     // ---- tiles q, k, v of every chunk: TMA, or copies that leave absent tokens zero ----
-    const int t = tid - kWorkWarps * 32, tiles = 3 * chunks;
+    const int t = tid - kWorkWarps * 32;
     const T* x = (const T*)p.x + (size_t)q0 * p.row_stride + (size_t)head * kDim;
-    for (int n = 0; n <= tiles; ++n) {                   // tile n is requested, tile n - 1 handed over
-      const int slot_n = n & 3;
-      if (n < tiles) {
-        const int which = n % 3, tok0 = n / 3 * kTok, off = which == 0 ? 0 : which == 1 ? p.k_off : p.v_off;
-        const uint32_t dst = s_ring + slot_n * kTileBytes;
-        bar_wait(&b_empty[slot_n], ((n >> 2) & 1) ^ 1, abort_flag, p.status);
-        if (tok0 + kTok <= qn) {
-          if (t == 0) {
-            const uint32_t bar = smem_u32(MEMORY ? &b_full[slot_n] : &b_raw[slot_n]);
-            mbar_expect_tx(bar, kTileBytes);
-            for (int i = 0; i < 2; ++i) tma_load_2d(dst + i * kSlab, &map_x, off + head * kDim + i * 64, q0 + tok0, bar);
-          }
+    for (int n = 0; n < 3 * chunks; ++n) {
+      const int which = n % 3, tok0 = n / 3 * kTok, off = which == 0 ? 0 : which == 1 ? p.k_off : p.v_off;
+      const uint32_t dst = s_ring + (n & 3) * kTileBytes, full = smem_u32(&b_full[n & 3]);
+      bar_wait(&b_empty[n & 3], ((n >> 2) & 1) ^ 1, abort_flag, p.status);
+      if (tok0 + kTok <= qn) {
+        if (t == 0) {
+          mbar_expect_tx(full, kTileBytes);
+          for (int i = 0; i < 2; ++i) tma_load_2d(dst + i * kSlab, &map_x, off + head * kDim + i * 64, q0 + tok0, full);
         } else {
-#pragma unroll 4
-          for (int e = t; e < kTok * 16; e += kLoaders<MEMORY>) {
-            const int r = e >> 4, c = e & 15;
-            const bool ok = tok0 + r < qn;
-            cp_async16_u32(dst + swizzled(r, c, kSlab), x + off + (size_t)(ok ? tok0 + r : 0) * p.row_stride + c * 8, ok);
-          }
-          cp_async_commit();
+          mbar_arrive(full);
         }
-      }
-      if (n == 0) continue;
-      const int before = n - 1, at_slot = before & 3;
-      const bool whole = before / 3 * kTok + kTok <= qn;
-      if (MEMORY && whole) {                             // TMA's bytes complete the phase; thread 0 has announced them
-        if (t != 0) mbar_arrive(smem_u32(&b_full[at_slot]));
         continue;
       }
-      if (whole) bar_wait(&b_raw[at_slot], (before >> 2) & 1, abort_flag, p.status);
-      else cp_async_wait<0>();
-      if (!MEMORY && before % 3 < 2) {
-        // (of a copied tile each thread works on the pieces that it copied; SiLU of zero is zero)
-        const uint32_t at = s_ring + at_slot * kTileBytes;
-#pragma unroll 2
-        for (int e = t; e < kTok * 16; e += kLoaders<MEMORY>) {
-          const uint32_t a = at + swizzled(e >> 4, e & 15, kSlab);
-          sts128(a, silu8<T>(lds128(a)));
-        }
+#pragma unroll 4
+      for (int e = t; e < kTok * 16; e += kLoaders) {
+        const int r = e >> 4, c = e & 15;
+        const bool ok = tok0 + r < qn;
+        cp_async16_u32(dst + swizzled(r, c, kSlab), x + off + (size_t)(ok ? tok0 + r : 0) * p.row_stride + c * 8, ok);
       }
+      cp_async_commit();
+      cp_async_wait<0>();
       fence_proxy_async();
-      mbar_arrive(smem_u32(&b_full[at_slot]));
+      mbar_arrive(full);
     }
   } else if (warp == kIssueWarp) {
     // ---- MMA issue ----
@@ -407,8 +408,12 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
     for (int i = 0; i < chunks; ++i) {
       const int nq = 3 * i, nk = nq + 1, nv = nq + 2, published = ctx > 0 ? i : i - 1;
       const uint32_t q = s_ring + (nq & 3) * kTileBytes, k = s_ring + (nk & 3) * kTileBytes, v = s_ring + (nv & 3) * kTileBytes;
-      bar_wait(&b_full[nq & 3], (nq >> 2) & 1, abort_flag, p.status);
-      bar_wait(&b_full[nk & 3], (nk >> 2) & 1, abort_flag, p.status);
+      if constexpr (MEMORY) {
+        bar_wait(&b_full[nq & 3], (nq >> 2) & 1, abort_flag, p.status);
+        bar_wait(&b_full[nk & 3], (nk >> 2) & 1, abort_flag, p.status);
+      } else {
+        bar_wait(&b_k, i & 1, abort_flag, p.status);
+      }
       __syncwarp();
       tc_fence_after();
       const uint32_t dq = desc_lo(q), dk = desc_lo(k);
