@@ -370,7 +370,8 @@ int launch_sbmm_prefill(const dz_sbmm_args& a, const void* xsrc, int sms, cudaSt
   p.num_kunits = (p.num_kblocks + 1) / 2;
   p.groups = a.N / kTileN;
   // One feature group only where their number is odd: with two an x tile serves both and two warps issue (12288 x 4096,
-  // 2048 tokens: 125 us, with one 148; 4096 x 4096, whose 192 tiles fill 1.3 waves: 68 and 70).
+  // 2048 tokens of one slot: 125 us, with one 148; 4096 x 4096, whose 192 tiles fill 1.3 waves: 68 and 70; with 48
+  // tiles, 513 tokens, still 64 against 69).
   p.F = p.groups % 2 == 0 ? 2 : 1;
   p.ldy = a.y_stride ? a.y_stride : a.N;
   p.qweight = (const uint8_t*)a.qweight; p.meta = (const uint8_t*)a.meta; p.scales = (const uint8_t*)a.scales;

@@ -80,7 +80,7 @@ def _convert_mapping(mapping: DeltaMapping, delta_index_to_id: List[Optional[int
     is_sorted = bool(n < 2 or (slots[1:] >= slots[:-1]).all())
     runs = None
     if is_sorted and n > ops.FUSED_MAX_TOKENS:
-        # prefill-sized batch: the runs of equal slots (host side), for the dequantise-once path
+        # prefill-sized batch: the runs of equal slots (host side)
         cuts = (torch.nonzero(slots[1:] != slots[:-1]).flatten() + 1).tolist()
         runs = [(int(slots[a]), a, b) for a, b in zip([0] + cuts, cuts + [n])]
     return (base_indices, sampler_indices, sampler_indices_padded, embeddings_indices,

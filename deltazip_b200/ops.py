@@ -10,8 +10,8 @@ PyTorch is used for memory and streams only -- every computation below runs in
 libdeltazip_b200.so, with one exception: for prefill-sized batches (more than
 FUSED_MAX_TOKENS rows) the plain dense product x W^T, the reference's F.linear
 (serving/vllm/model_executor/layers/linear.py:85-96), goes to the library GEMM
-(torch.matmul) once, and the library's kernel then adds the delta products into
-that result token block by token block.  The fused kernel streams W once per
+(torch.matmul) once, and the library's prompt kernel then adds the delta products into
+that result.  The fused kernel streams W once per
 block of 128 tokens, which is the right trade for decode batches and the wrong
 one for thousands of prompt tokens.
 """
@@ -29,10 +29,14 @@ from ._lib import SbmmArgs, check, lib
 
 # Largest batch (rows of x) that takes the fused kernel for base and delta products together.
 FUSED_MAX_TOKENS = 512
-# In a prefill-sized, sorted batch whose host-side run list is known (Segments.host_runs), a slot
-# with at least this many consecutive rows is dequantised once (dz_unpack) and multiplied by the
-# library GEMM, as the reference's PyTorch path does (deltazip/nn_modules/qlinear.py:266-330);
-# the SBMM kernel would expand the slot's codes once per 32-row window instead.
+# The delta products of such a batch are added by the prompt kernel, but for two cases of a sorted batch whose runs are
+# known on the host (Segments.host_runs) and have DENSE_RUN_TOKENS rows or more: there a slot is dequantised (dz_unpack)
+# and multiplied by the library GEMM, as the reference's PyTorch path does (deltazip/nn_modules/qlinear.py:266-330).
+# One is a single slot's rows over a matrix of at most DENSE_RUN_SIZE entries, too small to give every SM a tile (1280 x
+# 2048, 2048 rows: dequantised 38 us, prompt kernel 48; 4096 x 4096: 126 and 122; three slots of 1280 x 2048: 100 and
+# 48), the other a stack of more slots than the prompt kernel has tables for.
+PREFILL_MAX_SLOTS = 1024
+DENSE_RUN_SIZE = 1 << 23
 DENSE_RUN_TOKENS = 256
 # Decode attention of grouped query heads: keys a CTA should have where the keys are split.
 GROUPED_MIN_KEYS = 128
@@ -259,6 +263,8 @@ def sbmm(x: torch.Tensor, qweight_stacked: torch.Tensor, scales_stacked: torch.T
                 o2.copy_(base)
         runs = segments.host_runs
         if runs is not None and segments.sorted and \
+                (qweight_stacked.shape[0] > PREFILL_MAX_SLOTS or
+                 (n * k <= DENSE_RUN_SIZE and sum(slot >= 0 for slot, _, _ in runs) == 1)) and \
                 all(e - s >= DENSE_RUN_TOKENS for slot, s, e in runs if slot >= 0):
             o2 = out.reshape(-1, out.shape[-1]) if out.dim() != 2 else out
             for slot, s, e in runs:
