@@ -197,7 +197,8 @@ static_assert(mode_classes(false) * mode_r_per_class(2, false) <= kMaxR, "ring b
 
 // FULLK: K is a multiple of the 128-wide k-unit, so every unit has both half-tiles (the common
 // case; the tests on one half-tile in the loops fold away).
-template <int BITS, int DT, bool FULLK, bool WIDE>
+// COLS: 16, 64 or 128, the most columns of the token block.
+template <int BITS, int DT, bool FULLK, int COLS>
 __global__ void __launch_bounds__(kThreads, 1)
 sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_xc,
                const Params p) {
@@ -223,6 +224,7 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  constexpr bool WIDE = COLS > 64, narrow = COLS <= 16;
   constexpr int C = mode_classes(WIDE);
   constexpr int kDcols = mode_dcols(WIDE);
   constexpr int kWStages = mode_w_stages(WIDE), kXStages = mode_x_stages(WIDE);
@@ -785,10 +787,15 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       uint32_t csc[8];   // fp16 bit patterns of column chunk `wg`, two columns per word
 #pragma unroll
       for (int i = 0; i < 8; ++i) csc[i] = 0;
-      if (nwin > 0 && wg < p.cols / 16) {
+      // A warpgroup takes 16 columns, eight at a time, and every fourth chunk of them; of a block of 16 columns each takes
+      // four, so that the settling of its tiles -- the tail of calls of few tokens -- has all four at work and seven
+      // fragments to a round.
+      constexpr int cw = narrow ? 4 : 8;
+      if (nwin > 0 && (narrow || wg < p.cols / 16)) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int slot = s_slot[wg * 16 + i];
+          if (narrow && i >= 4) break;
+          const int slot = s_slot[wg * (narrow ? 4 : 16) + i];
           uint32_t v = 0;
           if (slot >= 0)
             v = *reinterpret_cast<const unsigned short*>(p.scales + (size_t)slot * p.sstride +
@@ -843,7 +850,7 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const uint32_t my_park = (uint32_t)(cta * 2 + (cta_first_fragment ? 0 : 1)) * (uint32_t)(p.cols * 128);
       // phase of the warpgroup's fix-up barrier (kept in shared memory between fragments)
       uint32_t fixpar = last ? s_fixpar[wg] : 0;
-      for (int c = wg; c < p.cols / 16; c += kNumWG) {
+      for (int c = wg; c < (narrow ? kNumWG : p.cols / 16); c += kNumWG) {
         if (nwin > 0 && c != wg) {   // second chunk of a wide token block: its scales are fetched here
 #pragma unroll
           for (int i = 0; i < 8; ++i) csc[i] = 0;
@@ -860,7 +867,8 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // eight columns at a time keep the epilogue's register needs below the main loop's
 #pragma unroll
         for (int hb = 0; hb < 2; ++hb) {
-          const int col = c * 16 + hb * 8;
+          if (narrow && hb > 0) break;
+          const int col = narrow ? c * 4 : c * 16 + hb * 8;   // (four columns: the other four loaded are not used)
           uint32_t v[8], d[8];
           if (p.delta_only) {
 #pragma unroll
@@ -881,21 +889,28 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           if (last) {
             // Sum over the tile's fragments in CTA order, this fragment's accumulators taking
             // their own place in that order.  Everything is summed out of shared memory: the
-            // thread's own 8 values go to slot 3 of the scratch, the other fragments' parked
+            // thread's own values go to the last slot of the scratch, the other fragments' parked
             // columns arrive three fragments at a time by bulk copies (one L2 round trip for
-            // 3 x 8 columns).  The scratch is the warpgroup's own two window buffers, idle
-            // until its next expansion.
+            // 3 x 8 columns; seven fragments of four).  The scratch is the warpgroup's own two
+            // window buffers, idle until its next expansion.
             const int my_f = cta - c_first;
             const uint32_t scr0 = s_winbuf + (wg < C ? wg : 2 * C + 2 * (wg - C)) * kWinBytes + r * 4;
             const uint32_t scr1 = scr0 + (wg < C ? C : 1) * kWinBytes;
             const uint32_t fixbar = smem_u32(&bar_fix[wg]);
+            constexpr int per = narrow ? 7 : 3;        // fragments of a round, one slot of cw x 512 bytes each
+            auto slot_at = [&](int ff) {           // slot ff of the scratch, this thread's row
+              const uint32_t off = (uint32_t)ff * cw * 512;
+              return off < 8192 ? scr0 + off : scr1 + (off - 8192);
+            };
+            const uint32_t own = slot_at(per);
             named_bar_sync(2 + wg, 128);   // nobody still reads the scratch (previous columns)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) sts32(scr1 + 4096 + i * 512, v[i]);
+            for (int i = 0; i < 8; ++i)
+              if (i < cw) sts32(own + i * 512, v[i]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0;   // from here on v is the running sum
-            for (int j = 0; j < nfrag - 1; j += 3) {
-              const int cnt = min(3, nfrag - 1 - j);
+            for (int j = 0; j < nfrag - 1; j += per) {
+              const int cnt = min(per, nfrag - 1 - j);
               if (j > 0) named_bar_sync(2 + wg, 128);
               if (wg_tid == 0) {
                 // the scratch was written by generic stores (shared), the parked partials by
@@ -903,48 +918,45 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 // copies, which go through the async proxy
                 fence_proxy_async();
                 asm volatile("fence.proxy.async.global;" ::: "memory");
-                mbar_expect_tx(fixbar, cnt * 4096);
+                mbar_expect_tx(fixbar, cnt * cw * 512);
 #pragma unroll
-                for (int ff = 0; ff < 3; ++ff) {
+                for (int ff = 0; ff < per; ++ff) {
                   if (ff >= cnt) break;
                   const int o = j + ff;   // o-th other fragment = fragment o, or o + 1 past this one
                   const int f = o + (o >= my_f ? 1 : 0);
                   // only the tile's first fragment can be its CTA's second parking slot
                   const uint32_t slot = (uint32_t)(c_first + f) * 2 + (f == 0 ? slot_first : 0);
                   const uint32_t off = (slot * (uint32_t)p.cols + (uint32_t)col) * 512u;
-                  bulk_load((ff < 2 ? scr0 : scr1) - r * 4 + (ff & 1) * 4096,
-                            reinterpret_cast<const uint8_t*>(p.partials) + off, 4096, fixbar);
+                  bulk_load(slot_at(ff) - r * 4, reinterpret_cast<const uint8_t*>(p.partials) + off, cw * 512, fixbar);
                 }
               }
               mbar_wait(fixbar, fixpar, abort_flag, p.status);
               fixpar ^= 1;
 #pragma unroll
-              for (int ff = 0; ff < 3; ++ff) {
+              for (int ff = 0; ff < per; ++ff) {
                 if (ff >= cnt) break;
                 if (j + ff == my_f) {   // this fragment comes right before its successor
 #pragma unroll
                   for (int i = 0; i < 8; ++i)
-                    v[i] = __float_as_uint(__uint_as_float(v[i]) +
-                                           __uint_as_float(lds32(scr1 + 4096 + i * 512)));
+                    if (i < cw) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(lds32(own + i * 512)));
                 }
-                const uint32_t src = (ff < 2 ? scr0 : scr1) + (ff & 1) * 4096;
+                const uint32_t src = slot_at(ff);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                  v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(lds32(src + i * 512)));
+                  if (i < cw) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(lds32(src + i * 512)));
               }
             }
             if (my_f == nfrag - 1) {
 #pragma unroll
               for (int i = 0; i < 8; ++i)
-                v[i] = __float_as_uint(__uint_as_float(v[i]) +
-                                       __uint_as_float(lds32(scr1 + 4096 + i * 512)));
+                if (i < cw) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(lds32(own + i * 512)));
             }
           }
           if (full_tile || last) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int prow = p.row0 + col + i;
-              if (prow < p.M) {
+              if (i < cw && prow < p.M) {
                 const int tok = s_tok[col + i];   // read in the prologue: no L2 round trip here
                 const size_t at = (size_t)tok * (size_t)p.ldy + n0 + r;
                 if (p.push_world == 0) {
@@ -958,10 +970,13 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-              __stcg(p.partials + (my_park + (uint32_t)((col + i) * 128 + r)), __uint_as_float(v[i]));
+              if (i < cw) __stcg(p.partials + (my_park + (uint32_t)((col + i) * 128 + r)), __uint_as_float(v[i]));
           }
         }
-        if (nwin > 0) tmem_st16_zero(lane_addr + kDcols + c * 16);   // D_delta restarts from zero
+        if (nwin > 0) {                            // D_delta restarts from zero
+          if (narrow) tmem_st4(lane_addr + kDcols + c * 4, 0, 0, 0, 0);
+          else tmem_st16_zero(lane_addr + kDcols + c * 16);
+        }
       }
       tmem_wait_st();
       tc_fence_before();
@@ -1037,7 +1052,7 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ x, const uint8_t* _
 // ---------------------------------------------------------------------------
 struct DeviceInfo {
   int sms = 0;
-  bool attr_set[16] = {};
+  bool attr_set[24] = {};
 };
 DeviceInfo& device_info(int dev) {
   static DeviceInfo info[64];
@@ -1147,16 +1162,13 @@ int launch_sbmm(const dz_sbmm_args& a, bool base_only, cudaStream_t st) {
     const size_t smem = (size_t)fixed + (size_t)p.nclass * p.r_per_class * rstage + 1024;
     const bool fullk = (a.K % kUnitK) == 0;
     using Kern = void (*)(const CUtensorMap, const CUtensorMap, const Params);
-    static const Kern kerns[16] = {
-        sbmm_tc_kernel<2, 0, false, false>, sbmm_tc_kernel<4, 0, false, false>,
-        sbmm_tc_kernel<2, 1, false, false>, sbmm_tc_kernel<4, 1, false, false>,
-        sbmm_tc_kernel<2, 0, true, false>,  sbmm_tc_kernel<4, 0, true, false>,
-        sbmm_tc_kernel<2, 1, true, false>,  sbmm_tc_kernel<4, 1, true, false>,
-        sbmm_tc_kernel<2, 0, false, true>,  sbmm_tc_kernel<4, 0, false, true>,
-        sbmm_tc_kernel<2, 1, false, true>,  sbmm_tc_kernel<4, 1, false, true>,
-        sbmm_tc_kernel<2, 0, true, true>,   sbmm_tc_kernel<4, 0, true, true>,
-        sbmm_tc_kernel<2, 1, true, true>,   sbmm_tc_kernel<4, 1, true, true>};
-    const int kidx = ((a.bits == 2) ? 0 : 1) + (dt ? 2 : 0) + (fullk ? 4 : 0) + (wide ? 8 : 0);
+#define DZ_KERNS(FULLK, COLS)                                                       \
+  sbmm_tc_kernel<2, 0, FULLK, COLS>, sbmm_tc_kernel<4, 0, FULLK, COLS>, sbmm_tc_kernel<2, 1, FULLK, COLS>, \
+      sbmm_tc_kernel<4, 1, FULLK, COLS>
+    static const Kern kerns[24] = {DZ_KERNS(false, 16), DZ_KERNS(true, 16), DZ_KERNS(false, 64),
+                                   DZ_KERNS(true, 64),  DZ_KERNS(false, 128), DZ_KERNS(true, 128)};
+#undef DZ_KERNS
+    const int kidx = ((a.bits == 2) ? 0 : 1) + (dt ? 2 : 0) + (fullk ? 4 : 0) + (p.cols <= 16 ? 0 : wide ? 16 : 8);
     Kern kern = kerns[kidx];
     if (!di.attr_set[kidx]) {
       DZ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
