@@ -43,7 +43,9 @@ GROUPED_MIN_KEYS = 128
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device.  (torch.cuda.current_stream builds a Stream object and looks at the
+    environment: 4 us, several times a call; a small model's decode pass spent a quarter of its time there.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*tensors):
@@ -129,7 +131,7 @@ class Segments:
         self.m = 0
         self.sorted = False
         # [(slot, first row, end row)] of a sorted batch when the caller knows it on the host
-        # (the slot manager does); None otherwise.  Only prefill-sized batches use it.
+        # (the slot manager does); None otherwise.  Only prefill-sized batches over very many slots use it.
         self.host_runs = None
 
     def build(self, indices: torch.Tensor, sorted_hint: Optional[bool] = None) -> "Segments":
@@ -167,6 +169,11 @@ class Segments:
 
 
 _workspaces = {}
+
+
+@functools.lru_cache(maxsize=4096)
+def _sbmm_workspace_bytes(m: int, n: int, k: int, tokens_sorted: bool) -> int:
+    return lib().dz_sbmm_workspace_bytes(m, n, k, int(tokens_sorted))
 
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
@@ -233,7 +240,7 @@ def sbmm(x: torch.Tensor, qweight_stacked: torch.Tensor, scales_stacked: torch.T
     goes to all tensor-parallel ranks' receive slots and `all_reduce_pushed` yields the sum;
     the call then returns None."""
     _need_cuda(x, qweight_stacked, scales_stacked, meta_stacked)
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     m, k = x2.shape
@@ -305,21 +312,18 @@ def sbmm(x: torch.Tensor, qweight_stacked: torch.Tensor, scales_stacked: torch.T
         raise ValueError(f"out must be a [{m}, {n}] {x.dtype} tensor with unit column stride")
     if m == 0:
         return out.reshape(*x.shape[:-1], n) if out.is_contiguous() else out
-    nbytes = lib().dz_sbmm_workspace_bytes(m, n, k, int(segments.sorted))
-    ws = _workspace(x.device, nbytes)
+    ws = _workspace(x.device, _sbmm_workspace_bytes(m, n, k, segments.sorted))
+    # in the order of the structure's fields: by name their assignment took as long as the launch
     args = SbmmArgs(
-        x=x2.data_ptr(), w_base=base_weight.data_ptr() if base_weight is not None else None,
-        qweight=qweight_stacked.data_ptr(), meta=meta_stacked.data_ptr(),
-        scales=scales_stacked.data_ptr(),
-        qweight_stride=qweight_stacked.stride(0) * 4, meta_stride=meta_stacked.stride(0) * 2,
-        scales_stride=scales_stacked.stride(0) * 2,
-        segments=segments.buf.data_ptr(), y=out2.data_ptr(),
-        M=m, N=n, K=k, num_slots=qweight_stacked.shape[0], bits=bits, dtype=_dtype_code(x),
-        tokens_sorted=int(segments.sorted),
-        flags=(_lib.DZ_SBMM_ACCUMULATE if accumulate else 0) | (_lib.DZ_SBMM_INPUTS_STABLE if stable else 0),
-        workspace=ws.data_ptr(), workspace_bytes=ws.numel(),
-        y_stride=max(out2.stride(0), n))
+        x2.data_ptr(), None if base_weight is None else base_weight.data_ptr(), qweight_stacked.data_ptr(),
+        meta_stacked.data_ptr(), scales_stacked.data_ptr(), qweight_stacked.stride(0) * 4, meta_stacked.stride(0) * 2,
+        scales_stacked.stride(0) * 2, segments.buf.data_ptr(), out2.data_ptr(), m, n, k, qweight_stacked.shape[0], bits,
+        _dtype_code(x), int(segments.sorted),
+        (_lib.DZ_SBMM_ACCUMULATE if accumulate else 0) | (_lib.DZ_SBMM_INPUTS_STABLE if stable else 0),
+        ws.data_ptr(), ws.numel(), max(out2.stride(0), n))
     check(getattr(lib(), _entry)(ctypes.byref(args), _stream()), _entry)
+    if out2 is out and x.dim() == 2:
+        return out
     return out.reshape(*x.shape[:-1], n) if out.is_contiguous() else out
 
 
@@ -347,7 +351,7 @@ def base_gemm(x: torch.Tensor, base_weight: torch.Tensor,
         out = torch.empty((m, n), dtype=x.dtype, device=x.device)
     if m == 0:
         return out.reshape(*x.shape[:-1], n)
-    ws = _workspace(x.device, lib().dz_sbmm_workspace_bytes(m, n, k, 1))
+    ws = _workspace(x.device, _sbmm_workspace_bytes(m, n, k, True))
     args = SbmmArgs(x=x2.data_ptr(), w_base=base_weight.data_ptr(), y=out.data_ptr(),
                     M=m, N=n, K=k, num_slots=0, bits=4, dtype=_dtype_code(x), tokens_sorted=1,
                     flags=_lib.DZ_SBMM_INPUTS_STABLE if stable else 0,
