@@ -10,7 +10,7 @@
 // With F = 2 an x tile serves 256 features: x is what a unit moves most of (45 KB of x to 6 KB of codes).  F = 1 is for
 // an odd number of feature groups.
 //
-// Measured on the four projections of a 7B decoder layer, 1999 tokens in seven runs, 4-bit: 4700 -> 1281 us with the
+// Measured on the four projections of a 7B decoder layer, 1999 tokens in seven runs, 4-bit: 4670 -> 1259 us with the
 // dense products (about 550 of them), against one pass of the decode kernel per 128 tokens.
 //
 // Roles: a TMA producer (x), a bulk-copy producer (packed stages), F MMA issuers, two warpgroups that expand, two
