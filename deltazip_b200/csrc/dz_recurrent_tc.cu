@@ -163,10 +163,16 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       const bool state = i > 0 || ctx > 0;
       const ChunkWeights& cw = s_cw[i & 1];
       if constexpr (MEMORY) bar_wait(&b_wfull[i & 1], (i >> 1) & 1, abort_flag, p.status);
-      bar_wait(&b_full[nv & 3], (nv >> 2) & 1, abort_flag, p.status);     // q and k came before it
-      __syncwarp();
+      // Each tile has a barrier of its own: copies complete in any order, and only a wait on a copy's own barrier makes
+      // its bytes visible.
+      if constexpr (MEMORY) {
+        for (int n = nq; n <= nv; ++n) bar_wait(&b_full[n & 3], (n >> 2) & 1, abort_flag, p.status);
+        __syncwarp();
+      }
       if constexpr (!MEMORY) {                           // q, k and v go through SiLU in place
         for (int n = nq; n <= nv; ++n) {
+          bar_wait(&b_full[n & 3], (n >> 2) & 1, abort_flag, p.status);
+          __syncwarp();
           const uint32_t at = s_ring + (n & 3) * kTileBytes;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -409,9 +415,11 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       const int nq = 3 * i, nk = nq + 1, nv = nq + 2, published = ctx > 0 ? i : i - 1;
       const uint32_t q = s_ring + (nq & 3) * kTileBytes, k = s_ring + (nk & 3) * kTileBytes, v = s_ring + (nv & 3) * kTileBytes;
       if constexpr (MEMORY) {
+        // the scores go where P V reads P: MMAs into different accumulators keep no order by themselves
+        if (i > 0) bar_wait(&b_pv, (i - 1) & 1, abort_flag, p.status);
         bar_wait(&b_full[nq & 3], (nq >> 2) & 1, abort_flag, p.status);
         bar_wait(&b_full[nk & 3], (nk >> 2) & 1, abort_flag, p.status);
-      } else {
+      } else {                                           // signalled by warps that have waited for P V
         bar_wait(&b_k, i & 1, abort_flag, p.status);
       }
       __syncwarp();
