@@ -88,12 +88,12 @@ grouped_decode_kernel(GroupedDecode p) {
                                              c * 32 + t * 8);
   }
   const int head = h0 + min(g, live - 1);
-  const float scale2 = p.scale * kLog2e;
+  // Scores are kept as they are, not times log2 e: a mask of the type's lowest value has to stay finite.
   const float* bias = p.bias ? p.bias + (size_t)head * p.bias_len : nullptr;
-  const float far_bias = bias ? bias[p.bias_len - 1] * kLog2e : 0.f;
+  const float far_bias = bias ? bias[p.bias_len - 1] : 0.f;
   // one warp of one split starts with the sink in its sum (which is kept per lane: the head's first one)
   const bool sink = p.sink && split == 0 && warp == 0;
-  float m = sink ? p.sink[head] * kLog2e : -INFINITY, l = sink && t == 0 ? 1.f : 0.f;
+  float m = sink ? p.sink[head] : -INFINITY, l = sink && t == 0 ? 1.f : 0.f;
   float o[16][4];                                              // [8 components][head g: 2, 2; its rounding's part: 2, 2]
 #pragma unroll
   for (int j = 0; j < 16; ++j)
@@ -125,17 +125,13 @@ grouped_decode_kernel(GroupedDecode p) {
         mma16816<T>(s[0], a0, k.x, k.y);
         mma16816<T>(s[1], a1, k.z, k.w);
       }
+      float b[2] = {far_bias, far_bias};
+      if (bias && len - 1 - (k0 + kTile - 1) < p.bias_len - 1) {         // distances that have a bias of their own
 #pragma unroll
-      for (int e = 0; e < 2; ++e) x[i][e] = fmaf(s[0][e] + s[1][e], scale2, far_bias);
-    }
-    if (bias && len - 1 - (k0 + kTile - 1) < p.bias_len - 1) { // distances that have a bias of their own
+        for (int e = 0; e < 2; ++e) b[e] = bias[min(max(len - 1 - (k0 + i * 8 + 2 * t + e), 0), p.bias_len - 1)];
+      }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int d = min(max(len - 1 - (k0 + i * 8 + 2 * t + e), 0), p.bias_len - 1);
-          x[i][e] += fmaf(bias[d], kLog2e, -far_bias);
-        }
+      for (int e = 0; e < 2; ++e) x[i][e] = fmaf(s[0][e] + s[1][e], p.scale, b[e]);
     }
     if (k0 + kTile > t1) {
 #pragma unroll
@@ -149,7 +145,7 @@ grouped_decode_kernel(GroupedDecode p) {
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float mn = fmaxf(m, mx), ms = mn == -INFINITY ? 0.f : mn;
     if (__any_sync(0xffffffffu, mn != m)) {
-      const float c = exp2f(m - ms);
+      const float c = __expf(m - ms);
       l *= c;
 #pragma unroll
       for (int j = 0; j < 16; ++j)
@@ -160,7 +156,7 @@ grouped_decode_kernel(GroupedDecode p) {
     uint32_t a[4];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const float w0 = exp2f(x[i][0] - ms), w1 = exp2f(x[i][1] - ms);
+      const float w0 = __expf(x[i][0] - ms), w1 = __expf(x[i][1] - ms);
       l += w0 + w1;
       split_pair<T>(w0, w1, a[2 * i], a[2 * i + 1]);
     }
@@ -203,7 +199,7 @@ grouped_decode_kernel(GroupedDecode p) {
     for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, s_m[w][h]);
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float c = s_m[w][h] == -INFINITY ? 0.f : exp2f(s_m[w][h] - mm);
+      const float c = s_m[w][h] == -INFINITY ? 0.f : __expf(s_m[w][h] - mm);
       const float4 v = *reinterpret_cast<const float4*>(smem + w * kRingBytes + (size_t)i * 4);
       sum += s_l[w][h] * c;
       a[0] += v.x * c;
@@ -240,7 +236,7 @@ grouped_decode_kernel(GroupedDecode p) {
     for (int s = 0; s < p.splits; ++s) {
       const float2 w = __ldcg(&ml[at + s]);
       const float4 v = __ldcg(reinterpret_cast<const float4*>(p.partial + (at + s) * kGroupedDim + d));
-      const float c = w.x == -INFINITY ? 0.f : exp2f(w.x - mm);
+      const float c = w.x == -INFINITY ? 0.f : __expf(w.x - mm);
       sum += w.y * c;
       a[0] += v.x * c;
       a[1] += v.y * c;

@@ -84,3 +84,38 @@ def test_window(heads, kvh, window, splits, extra, dtype):
             at = tables[i].long()[pos // BLOCK % ring] * BLOCK + pos % BLOCK
             b = bias[:, (n - 1 - pos).clamp(max=39)] if extra else None
             check(out[i], reference(qkv[i, :heads * 128].view(heads, 128), k[at], v[at], 0.11, b, sink), dtype)
+
+
+@pytest.mark.parametrize("mask", [float("-inf"), torch.finfo(torch.float32).min, -1e9, -1e6, -1e4])
+@pytest.mark.parametrize("splits", [1, 4])
+def test_bias_that_masks_far_keys(mask, splits):
+    """The last bias of the table, which all farther keys share, hides them: near keys keep their scores."""
+    from deltazip_b200 import ops
+    heads, kvh, dtype, length = 8, 1, torch.float16, 40
+    qkv, k, v, tables = batch(kvh, heads, dtype, 3, -(-max(LENS) // BLOCK), LENS)
+    bias = torch.randn((heads, length), generator=torch.Generator("cuda").manual_seed(4), device="cuda")
+    bias[:, 21:] = mask                            # hidden beyond distance 20, the shared entry among them
+    starts = torch.arange(len(LENS) + 1, dtype=torch.int32, device="cuda")
+    ctx = torch.tensor([n - 1 for n in LENS], dtype=torch.int32, device="cuda")
+    out = ops.window_attention(qkv, k, v, tables, starts, ctx, 1, True, heads, BLOCK, 0.3, 0, bias, splits, None)
+    for i, n in enumerate(LENS):
+        pos = torch.arange(n, device="cuda")
+        at = tables[i].long()[pos // BLOCK] * BLOCK + pos % BLOCK
+        b = bias[:, (n - 1 - pos).clamp(max=length - 1)]
+        check(out[i], reference(qkv[i, :heads * 128].view(heads, 128), k[at], v[at], 0.3, b), dtype)
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+def test_every_key_masked_by_the_lowest_value(splits):
+    """Finite masks over all keys leave equal weights: the mean of the values."""
+    from deltazip_b200 import ops
+    heads, kvh, dtype = 8, 1, torch.float16
+    qkv, k, v, tables = batch(kvh, heads, dtype, 3, -(-max(LENS) // BLOCK), LENS)
+    bias = torch.full((heads, 40), torch.finfo(torch.float32).min, device="cuda")
+    starts = torch.arange(len(LENS) + 1, dtype=torch.int32, device="cuda")
+    ctx = torch.tensor([n - 1 for n in LENS], dtype=torch.int32, device="cuda")
+    out = ops.window_attention(qkv, k, v, tables, starts, ctx, 1, True, heads, BLOCK, 0.3, 0, bias, splits, None)
+    for i, n in enumerate(LENS):
+        pos = torch.arange(n, device="cuda")
+        at = tables[i].long()[pos // BLOCK] * BLOCK + pos % BLOCK
+        check(out[i].view(heads, 128), v[at, 0].double().mean(0).expand(heads, 128), dtype)
