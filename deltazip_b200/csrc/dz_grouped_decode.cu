@@ -3,17 +3,19 @@
 //
 // Bound: the cache's bytes.  On CUDA cores eight heads cost 16 multiply-adds and conversions per byte, which
 // held the kernel at a seventh of the copy bandwidth; here the heads are the rows of a warp MMA, so a 16-key tile
-// costs 32 of them whatever the head count.
+// costs 48 of them whatever the head count.
 //   scores   S[heads, 8 keys] += Q K^T: the eight heads are rows 0-7 of the 16-row operand.  The order of the 128
 //            products of a score is free, so a lane's 16-byte piece of a key row serves two MMAs as it lies.
-//   output   O[heads, 128] += P V: rows 0-7 carry the weights rounded to 16 bits, rows 8-15 what the rounding took
-//            away, so one MMA adds both halves of a 32-bit weight; V comes transposed by ldmatrix.
+//   output   O[heads, 128] += P V: a 32-bit weight is the sum of three 16-bit parts, hi, mid and lo.  Rows 0-7 of two
+//            MMAs carry half of hi each, rows 8-15 mid and lo; V comes transposed by ldmatrix.  (No row of an MMA
+//            mixes hi with a part that may be zero: an infinity in V stays one.)
 // A CTA is four warps over the keys of one (sequence, key/value head, split), 16 keys per warp and step, each warp
 // with a ring of three tiles of its own (cp.async, no barrier but the warp's): two CTAs of 96 KB per SM keep 128 KB
 // of the cache in flight.  Chunks of a row are stored in an order that depends on the row (swizzle), so that
 // neither the 16-byte reads of K nor ldmatrix meet a bank twice.
-// Measured, 64 sequences x 64 query heads on 8, 938 keys in the mean (249 MB, 38 us at the copy bandwidth): 51 us, the
-// form on CUDA cores 272; 32 heads on 8, 2560 keys: 0.85 of the copy bandwidth.
+// Measured, 64 sequences x 64 query heads on 8, 938 keys in the mean (246 MB, 38 us at the copy bandwidth): 50.8 us
+// (weights of two parts, 16 to 22 bits: 47.3), the form on CUDA cores 272; 32 heads on 8, 2560 keys: 0.85 of the copy
+// bandwidth.
 #include "dz_grouped_decode.cuh"
 
 namespace dz {
@@ -28,6 +30,19 @@ static_assert(kRingBytes >= kGroupedHeads * kGroupedDim * 4, "a warp's ring also
 // Where 16-byte chunk c of row r lies: rows r, r + 1 in different halves of the banks, any eight consecutive
 // rows in eight different chunks.
 __device__ __forceinline__ int chunk_at(int r, int c) { return r * kRowBytes + ((c ^ ((r & 1) << 2 | (r >> 1 & 3))) << 4); }
+
+// Two weights in [0, 1] times `kScale` as half + half + mid + lo: 24 bits, all of a weight's (fp16: of weights above
+// 2^-16; below, what is lost is at most 2^-40, which no sum of weights around 1 can hold).
+template <typename T> constexpr float kScale = 1.f;
+template <> constexpr float kScale<__half> = 32768.f;
+template <typename T>
+__device__ __forceinline__ void split_weights(float a, float b, uint32_t& half, uint32_t& mid, uint32_t& lo) {
+  a *= 0.5f * kScale<T>;
+  b *= 0.5f * kScale<T>;
+  half = Cvt<T>::down(a, b);
+  const float2 h = Cvt<T>::up(half);
+  split_pair<T>(2.f * (a - h.x), 2.f * (b - h.y), mid, lo);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kWarps * 32, 2)
@@ -55,15 +70,15 @@ grouped_decode_kernel(GroupedDecode p) {
     const int k = min(t0 + tile * kTile + (lane & 15), t1 - 1), b = k / p.block_size;
     return ((uint32_t)table[b % p.ring_blocks] * p.block_size + (k - b * p.block_size)) * p.kv_heads + kvh;
   };
-  auto issue = [&](int stage, uint32_t row) {
-    const int c = lane & 15;
+  auto issue = [&](int stage, int tile, uint32_t row) {
+    const int c = lane & 15, keys = t1 - t0 - tile * kTile;    // values past the end are zero, as their weights are
 #pragma unroll
     for (int j = 0; j < kTile / 2; ++j) {
       const int r = 2 * j + (lane >> 4);
       const size_t at = (size_t)__shfl_sync(0xffffffffu, row, r) * kGroupedDim + c * 8;
       uint8_t* dst = ring + stage * kStageBytes + chunk_at(r, c);
       cp_async16(dst, kc + at, true);
-      cp_async16(dst + kHalfStage, vc + at, true);
+      cp_async16(dst + kHalfStage, vc + at, r < keys);
     }
   };
   const int tiles = t1 > t0 ? (t1 - t0 + kTile - 1) / kTile : 0;
@@ -73,7 +88,7 @@ grouped_decode_kernel(GroupedDecode p) {
   for (int s = 0; s < kStages - 1; ++s) {
     const int tile = warp + s * kWarps;
     if (tile < tiles) {
-      issue(s, next);
+      issue(s, tile, next);
       if (tile + kWarps < tiles) next = row_of(tile + kWarps);
     }
     cp_async_commit();
@@ -94,7 +109,7 @@ grouped_decode_kernel(GroupedDecode p) {
   // one warp of one split starts with the sink in its sum (which is kept per lane: the head's first one)
   const bool sink = p.sink && split == 0 && warp == 0;
   float m = sink ? p.sink[head] : -INFINITY, l = sink && t == 0 ? 1.f : 0.f;
-  float o[16][4];                                              // [8 components][head g: 2, 2; its rounding's part: 2, 2]
+  float o[16][4];                                              // [8 components][head g: 2 of hi; 2 of mid and lo]
 #pragma unroll
   for (int j = 0; j < 16; ++j)
 #pragma unroll
@@ -107,7 +122,7 @@ grouped_decode_kernel(GroupedDecode p) {
     {
       const int ahead = tile + (kStages - 1) * kWarps;
       if (ahead < tiles) {
-        issue(stage == 0 ? kStages - 1 : stage - 1, next);
+        issue(stage == 0 ? kStages - 1 : stage - 1, ahead, next);
         if (ahead + kWarps < tiles) next = row_of(ahead + kWarps);
       }
       cp_async_commit();
@@ -153,12 +168,13 @@ grouped_decode_kernel(GroupedDecode p) {
         for (int e = 0; e < 4; ++e) o[j][e] *= c;
       m = mn;
     }
-    uint32_t a[4];
+    uint32_t a[4], a2[4];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const float w0 = __expf(x[i][0] - ms), w1 = __expf(x[i][1] - ms);
       l += w0 + w1;
-      split_pair<T>(w0, w1, a[2 * i], a[2 * i + 1]);
+      split_weights<T>(w0, w1, a[2 * i], a[2 * i + 1], a2[2 * i + 1]);
+      a2[2 * i] = a[2 * i];
     }
     const uint8_t* vs = ks + kHalfStage;
 #pragma unroll
@@ -167,6 +183,8 @@ grouped_decode_kernel(GroupedDecode p) {
       ldsm4_t(b, vs + chunk_at(lane & 15, 2 * j + (lane >> 4)));
       mma16816<T>(o[2 * j], a, b[0], b[1]);
       mma16816<T>(o[2 * j + 1], a, b[2], b[3]);
+      mma16816<T>(o[2 * j], a2, b[0], b[1]);
+      mma16816<T>(o[2 * j + 1], a2, b[2], b[3]);
     }
     stage = stage == kStages - 1 ? 0 : stage + 1;
   }
@@ -175,9 +193,11 @@ grouped_decode_kernel(GroupedDecode p) {
   l += __shfl_xor_sync(0xffffffffu, l, 2);
   __syncwarp();                                                // the warp's ring becomes its output [heads, 128]
   float* own = reinterpret_cast<float*>(ring);
+  // where the values held an infinity, hi's products are the result and the other parts' may be anything
+  auto whole = [](float hi, float rest) { return (isfinite(hi) ? hi + rest : hi) * (1.f / kScale<T>); };
 #pragma unroll
   for (int j = 0; j < 16; ++j)
-    *reinterpret_cast<float2*>(own + g * kGroupedDim + j * 8 + 2 * t) = make_float2(o[j][0] + o[j][2], o[j][1] + o[j][3]);
+    *reinterpret_cast<float2*>(own + g * kGroupedDim + j * 8 + 2 * t) = make_float2(whole(o[j][0], o[j][2]), whole(o[j][1], o[j][3]));
   if (t == 0) {
     s_m[warp][g] = m;
     s_l[warp][g] = l;
@@ -188,8 +208,8 @@ grouped_decode_kernel(GroupedDecode p) {
   const size_t column = (size_t)seq * p.heads + h0;
   float2* const ml = reinterpret_cast<float2*>(p.partial + (size_t)gridDim.y * p.heads * p.splits * kGroupedDim);
   auto store = [&](int h, int d, const float (&a)[4], float sum) {
-    const float inv = p.empty_is_zero && !(sum > 0.f) ? 0.f : 1.f / sum;
-    uint2 v = make_uint2(Cvt<T>::down(a[0] * inv, a[1] * inv), Cvt<T>::down(a[2] * inv, a[3] * inv));
+    uint2 v = make_uint2(Cvt<T>::down(a[0] / sum, a[1] / sum), Cvt<T>::down(a[2] / sum, a[3] / sum));
+    if (p.empty_is_zero && !(sum > 0.f)) v = make_uint2(0, 0);
     *reinterpret_cast<uint2*>((T*)p.out + (column + h) * kGroupedDim + d) = v;
   };
   for (int i = threadIdx.x * 4; i < live * kGroupedDim; i += kWarps * 32 * 4) {

@@ -2,7 +2,7 @@
 lengths around its 16-key tiles, four warps and splits, group sizes that fill the eight MMA rows or not, windows,
 distance bias and sinks.
 
-Tolerance: scores and sums are 32-bit and a weight enters as two 16-bit parts, so what is left is the output's
+Tolerance: scores, sums and weights (three 16-bit parts) are 32-bit, so what is left is the output's
 rounding, at most half a unit in the last place: 2^-11 (fp16) or 2^-8 (bf16) of every element; twice that for the
 relative 2-norm."""
 import pytest
@@ -119,3 +119,58 @@ def test_every_key_masked_by_the_lowest_value(splits):
         pos = torch.arange(n, device="cuda")
         at = tables[i].long()[pos // BLOCK] * BLOCK + pos % BLOCK
         check(out[i].view(heads, 128), v[at, 0].double().mean(0).expand(heads, 128), dtype)
+
+
+def test_weights_keep_32_bits():
+    """bf16, four keys a sequence whose products with the weights cancel down to 2^-16 of themselves, so that the output's
+    own rounding is out of the way.  Error allowed against the sum of absolute products: 2^-19.5, from two units of the
+    exponential and three 32-bit sums (2^-21); a weight of two 16-bit parts is off by up to 2^-18."""
+    from deltazip_b200 import ops
+    n, heads, dtype = 64, 8, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q = torch.randn((n, 1, 128), generator=g, device="cuda").to(dtype)
+    k = torch.randn((n * BLOCK, 1, 128), generator=g, device="cuda").to(dtype)
+    v = (1 + torch.rand((n, BLOCK, 128), generator=g, device="cuda")).to(dtype)
+    w = torch.einsum("nd,nkd->nk", q[:, 0].double(), k.view(n, BLOCK, 128)[:, :4].double()).mul(128 ** -0.5).softmax(1)
+    for key in (2, 3):                             # each takes away what the keys before it leave
+        v[:, key] = (-(w[:, :key, None] * v[:, :key].double()).sum(1) / w[:, key, None]).to(dtype)
+    qkv = torch.cat([q.expand(n, heads, 128).reshape(n, -1), torch.zeros((n, 256), device="cuda", dtype=dtype)], 1).contiguous()
+    tables, lens = (t.int().cuda() for t in (torch.arange(n)[:, None], torch.full((n,), 4)))
+    out = ops.paged_attention_decode(qkv, k, v.reshape(-1, 1, 128), tables.contiguous(), lens, heads, 1, BLOCK, 128 ** -0.5)
+    parts = w[:, :, None] * v[:, :4].double()
+    err = (out.view(n, heads, 128).double() - parts.sum(1)[:, None]).abs() / parts.abs().sum(1)[:, None]
+    assert float(err.max()) <= 2.0 ** -19.5, float(err.max())
+
+
+def test_small_weights_add_up():
+    """fp16: 6000 keys at 2^-26 of the largest weight each, alone in having values."""
+    from deltazip_b200 import ops
+    heads, n, dtype = 4, 6000, torch.float16
+    blocks = -(-n // BLOCK)
+    v = torch.ones((blocks * BLOCK, 1, 128), device="cuda", dtype=dtype)
+    v[n - 1] = 0
+    bias = torch.tensor([[0.0, -26 * 0.6931471805599453]] * heads, device="cuda")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    out = ops.window_attention(torch.zeros((1, (heads + 2) * 128), device="cuda", dtype=dtype), torch.zeros_like(v), v,
+                               torch.arange(blocks, dtype=torch.int32, device="cuda")[None], i32([0, 1]), i32([n - 1]), 1, True,
+                               heads, BLOCK, 1.0, 0, bias, 1, None)
+    tail = (n - 1) * 2.0 ** -26
+    check(out[0], torch.full_like(out[0], tail / (1 + tail), dtype=torch.float64), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("length,key", [(16, 3), (21, 20), (70, 69), (70, 5)])
+def test_infinities_among_the_values(length, key, dtype):
+    """An infinite component of a value gives that infinity, and leaves the other components alone; values that repeat
+    behind a sequence's end do not count."""
+    from deltazip_b200 import ops
+    heads = 8
+    qkv, k, v, tables = batch(1, heads, dtype, length, 5, [length])
+    v[int(tables[0, key // BLOCK]) * BLOCK + key % BLOCK, 0, 7] = float("inf")
+    v[int(tables[0, key // BLOCK]) * BLOCK + key % BLOCK, 0, 12] = float("-inf")
+    out = ops.paged_attention_decode(qkv, k, v, tables, torch.tensor([length], dtype=torch.int32, device="cuda"), heads, 1, BLOCK, 0.02)
+    at = (tables[0].long()[:, None] * BLOCK + torch.arange(BLOCK, device="cuda")).flatten()[:length]
+    want = reference(qkv[0, :heads * 128].view(heads, 128), k[at], v[at], 0.02)
+    bad = torch.isinf(want)
+    assert torch.equal(torch.where(bad, out[0].double(), 0), torch.where(bad, want, 0)) and int(bad.sum()) == 2 * heads
+    check(out[0][~bad], want[~bad], dtype)
