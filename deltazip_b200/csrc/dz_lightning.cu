@@ -549,7 +549,8 @@ int dz_lightning_chunk_supported(int dim, int vdim, int dtype) {
 }
 
 size_t dz_lightning_workspace_bytes(int rows, int num_seqs, int heads, int vdim, int chunkwise) {
-  if (rows <= 0 || num_seqs <= 0 || heads <= 0 || vdim <= 0 || chunkwise) return 0;
+  if (rows <= 0 || num_seqs <= 0 || heads <= 0 || vdim <= 0) return 0;
+  if (chunkwise) return kRecStatusBytes;
   return kTicketBytes + (size_t)rows * heads * vdim * 4;
 }
 
@@ -582,12 +583,13 @@ int dz_lightning(const dz_lightning_args* a, void* stream) {
   if (!dz_lightning_chunk_supported(a->dim, a->vdim, a->dtype)) return DZ_ERR_UNSUPPORTED;
   if (a->row_stride % 8 || a->k_off % 8 || a->v_off % 8 || !aligned16(a->x) || !aligned16(a->out)) return DZ_ERR_ALIGNMENT;
   int rc = DZ_OK;
-  if (a->dim == 128 && a->vdim == 128 && a->row_stride < (1ll << 31)) {
+  // (its waits are bounded: without a place to report one that ran out the kernel that has none is taken)
+  if (a->dim == 128 && a->vdim == 128 && a->row_stride < (1ll << 31) && a->workspace && a->workspace_bytes >= kRecStatusBytes) {
     RecurrentParams r = {};
     r.x = a->x; r.row_stride = a->row_stride; r.rows = a->rows; r.k_off = a->k_off; r.v_off = a->v_off;
     r.out = a->out; r.S = a->S; r.slots = a->slots; r.q_starts = a->q_starts; r.ctx_lens = a->ctx_lens;
     r.heads = a->heads; r.powers = a->powers;
-    r.status = recurrent_status(a->workspace, a->workspace_bytes, 0);
+    r.status = (int*)a->workspace;
     rc = launch_recurrent_tc(r, false, a->dtype, a->num_seqs, st);
     if (rc) return rc;
     DZ_DISPATCH16(a->dtype, return (run_norm<T, T>(p, (const T*)p.out, a->rows, st)));

@@ -642,7 +642,7 @@ int dz_mlstm_chunk_supported(int dim, int vdim, int dtype) {
 }
 
 size_t dz_mlstm_workspace_bytes(int num_seqs, int heads) {
-  return num_seqs > 0 && heads > 0 ? (size_t)num_seqs * heads * 4 : 0;
+  return num_seqs > 0 && heads > 0 ? kRecStatusBytes + (size_t)num_seqs * heads * 4 : 0;
 }
 
 int dz_mlstm(const dz_mlstm_args* a, void* stream) {
@@ -676,14 +676,15 @@ int dz_mlstm(const dz_mlstm_args* a, void* stream) {
     r.out = a->out; r.S = a->S; r.slots = a->slots; r.q_starts = a->q_starts; r.ctx_lens = a->ctx_lens;
     r.heads = a->heads; r.pre_if = a->pre_if; r.b_if = a->b_if; r.cap = a->cap; r.scale = a->scale;
     r.n = a->n; r.m = a->m; r.norm_w = a->norm_weight; r.eps = a->eps;
-    r.status = recurrent_status(a->workspace, a->workspace_bytes, dz_mlstm_workspace_bytes(a->num_seqs, a->heads));
+    r.status = (int*)a->workspace;
     return launch_recurrent_tc(r, true, a->dtype, a->num_seqs, st);
   }
   const int dimp = (a->dim + 15) / 16 * 16;
   int rc = DZ_OK;
+  int* const tickets = (int*)((uint8_t*)a->workspace + kRecStatusBytes);
   const bool wide = a->vdim > 32 && dimp <= 256 && chunk_smem(dimp, 64) <= kMaxDynSmem;
-  DZ_DISPATCH16(a->dtype, rc = wide ? run_chunk<T, 64>(p, a->num_seqs, dimp, (int*)a->workspace, st)
-                                    : run_chunk<T, 32>(p, a->num_seqs, dimp, (int*)a->workspace, st));
+  DZ_DISPATCH16(a->dtype, rc = wide ? run_chunk<T, 64>(p, a->num_seqs, dimp, tickets, st)
+                                    : run_chunk<T, 32>(p, a->num_seqs, dimp, tickets, st));
   if (rc) return rc;
   const unsigned blocks = (unsigned)(((int64_t)a->rows * a->heads + 7) / 8);
   DZ_DISPATCH16(a->dtype,

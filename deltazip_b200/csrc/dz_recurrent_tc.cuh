@@ -16,7 +16,7 @@ struct RecurrentParams {
   const int* q_starts;
   const int* ctx_lens;
   int heads;
-  int* status;                           // first error, or nullptr
+  int* status;                           // first error: the first word of the call's workspace
   // matrix memory: gates, denominator, head norm and output gate
   const float* pre_if;                   // [rows, 2 heads]
   const float* b_if;
@@ -28,12 +28,7 @@ struct RecurrentParams {
   const float* powers;                   // [heads, 65] w^0 ... w^64
 };
 
-// The status word of a chunkwise call: the last 16 bytes of a workspace that has them behind the `used` ones.
-inline int* recurrent_status(void* workspace, size_t bytes, size_t used) {
-  if (!workspace || bytes < used + 32) return nullptr;
-  const uintptr_t end = reinterpret_cast<uintptr_t>(workspace) + bytes - 16;
-  return reinterpret_cast<int*>(end & ~(uintptr_t)15);
-}
+constexpr size_t kRecStatusBytes = 256;  // workspace of a chunkwise call: [status word | tickets]
 
 int launch_recurrent_tc(const RecurrentParams& p, bool matrix_memory, int dtype, int num_seqs, cudaStream_t st);
 

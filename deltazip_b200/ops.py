@@ -193,20 +193,16 @@ def read_status(device=None) -> int:
     kernels leave in the current stream's workspaces (0 = ok, DZ_ERR_TIMEOUT = a bounded device-side wait ran
     out, DZ_ERR_INVALID_ARG = a wrong `tokens_sorted` promise).  Synchronises."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    found, words = 0, []
-    for ws in (_workspaces.get((device.index, _stream())),
-               _scratch.get(("window_attention", device.index, _stream())),
-               _scratch.get(("status", device.index, _stream()))):
-        if ws is not None:
-            words.append(ws.data_ptr())
-    for kind in ("mlstm", "lightning_chunk"):
-        ws = _scratch.get((kind, device.index, _stream()))
-        if ws is not None:
-            words.append((ws.data_ptr() + ws.numel() - 16) & ~15)
+    found = 0
+    words = [_workspaces.get((device.index, _stream()))]
+    for kind in _STATUS_FIRST:
+        key = (kind, device.index, _stream())
+        words += [_scratch.get(key), *_replaced.pop(key, ())]
     for word in words:
-        host = ctypes.c_int(0)
-        check(lib().dz_read_status(word, _stream(), ctypes.byref(host)), "dz_read_status")
-        found = found or host.value
+        if word is not None:
+            host = ctypes.c_int(0)
+            check(lib().dz_read_status(word.data_ptr(), _stream(), ctypes.byref(host)), "dz_read_status")
+            found = found or host.value
     return found
 
 
@@ -644,9 +640,10 @@ def paged_attention_decode(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: to
 # blocks, matrix-memory recurrence.  16-bit or 32-bit activations, any sizes.
 # ---------------------------------------------------------------------------
 
-STATUS_TAIL = 32                        # scratch of a chunkwise recurrence ends with its status word (in the last 16 bytes)
 ACTIVATIONS = {"silu": _lib.DZ_ACT_SILU, "gelu_tanh": _lib.DZ_ACT_GELU_TANH, "relu2": _lib.DZ_ACT_RELU2}
 _scratch = {}
+_STATUS_FIRST = ("window_attention", "status", "mlstm", "lightning_chunk")      # scratch that starts with a status word
+_replaced = {}                          # such scratch that a larger one took the place of, until its word is read
 
 
 def _zeroed_scratch(kind: str, device, nbytes: int) -> Optional[torch.Tensor]:
@@ -657,6 +654,10 @@ def _zeroed_scratch(kind: str, device, nbytes: int) -> Optional[torch.Tensor]:
     key = (kind, device.index, _stream())
     buf = _scratch.get(key)
     if buf is None or buf.numel() < nbytes:
+        if kind in _STATUS_FIRST:
+            nbytes = 1 << (nbytes - 1).bit_length()      # all replaced ones together are smaller
+            if buf is not None:
+                _replaced.setdefault(key, []).append(buf)
         buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
         _scratch[key] = buf
     return buf
@@ -929,10 +930,8 @@ def lightning(x: torch.Tensor, powers: torch.Tensor, norm_weight: torch.Tensor, 
     if powers.shape != (heads, LIGHTNING_POWERS) or powers.dtype != torch.float32 or not powers.is_contiguous():
         raise ValueError("powers must be a contiguous float32 [heads, 65]")
     out = torch.empty((rows, heads * vdim), dtype=x.dtype, device=x.device)
-    if chunkwise:
-        ws = _zeroed_scratch("lightning_chunk", x.device, STATUS_TAIL)
-    else:
-        ws = _zeroed_scratch("lightning", x.device, lib().dz_lightning_workspace_bytes(rows, seqs, heads, vdim, 0))
+    ws = _zeroed_scratch("lightning_chunk" if chunkwise else "lightning", x.device,
+                         lib().dz_lightning_workspace_bytes(rows, seqs, heads, vdim, int(chunkwise)))
     args = _lib.LightningArgs(
         x=x.data_ptr(), row_stride=x.stride(0), k_off=heads * dim, v_off=2 * heads * dim,
         g_off=2 * heads * dim + heads * vdim, powers=powers.data_ptr(), norm_weight=norm_weight.data_ptr(),
@@ -960,7 +959,7 @@ def mlstm(x: torch.Tensor, h: torch.Tensor, w_if: torch.Tensor, b_if: torch.Tens
         raise ValueError("slots / q_starts / ctx_lens must be contiguous int32")
     out = torch.empty((rows, heads * vdim), dtype=x.dtype, device=x.device)
     pre = matmul_f32(h, w_if) if chunkwise else None
-    ws = _zeroed_scratch("mlstm", x.device, lib().dz_mlstm_workspace_bytes(seqs, heads) + STATUS_TAIL) if chunkwise else None
+    ws = _zeroed_scratch("mlstm", x.device, lib().dz_mlstm_workspace_bytes(seqs, heads)) if chunkwise else None
     args = _lib.MlstmArgs(
         x=x.data_ptr(), row_stride=x.stride(0), k_off=heads * dim, v_off=2 * heads * dim,
         g_off=2 * heads * dim + heads * vdim, h=h.data_ptr(), w_if=w_if.data_ptr(), b_if=b_if.data_ptr(),

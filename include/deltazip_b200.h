@@ -389,8 +389,10 @@ int dz_kv_append(const void* qkv, int64_t row_stride, int k_off, int k_width, in
  * state pools S [slots, heads, dim, vdim], n [slots, heads, dim], m [slots, heads] are 32-bit and
  * updated in place; a sequence with ctx_lens 0 starts from zero without reading its slot.
  * chunkwise = 0: token after token, gates from h [rows, width] and w_if [2 heads, width] (w_i, w_f);
- * chunkwise = 1 (dz_mlstm_chunk_supported): 64 tokens at a time, gates from pre_if [rows, 2 heads];
- * the workspace must be zero-filled once before its first use.
+ * chunkwise = 1 (dz_mlstm_chunk_supported): 64 or 128 tokens at a time, gates from pre_if [rows, 2 heads];
+ * the workspace (dz_mlstm_workspace_bytes) must be zero-filled once before its first use.  Its first word
+ * is the status word (dz_read_status): DZ_ERR_TIMEOUT where a bounded wait of the kernel for heads of
+ * 128 x 128 ran out; outputs and states of that call are then not to be used.
  */
 typedef struct dz_mlstm_args {
   const void* x;
@@ -482,8 +484,10 @@ int dz_latent_attention(const dz_latent_attention_args* args, void* stream);
  * (plain weight) * sigmoid(g).  Rows are [q | k | v | g] (heads * dim, heads * dim, heads * vdim,
  * heads * vdim); S [slots, heads, dim, vdim] is 32-bit and updated in place; a sequence with ctx_lens 0
  * starts from zero without reading its slot.  powers [heads, 65]: decay^0 ... decay^64.
- * chunkwise = 1 (dz_lightning_chunk_supported): 64 tokens at a time.  The workspace must be zero-filled
- * once before its first use.
+ * chunkwise = 1 (dz_lightning_chunk_supported): 64 or 128 tokens at a time.  The workspace
+ * (dz_lightning_workspace_bytes) must be zero-filled once before its first use.  With chunkwise = 1 its
+ * first word is the status word, as dz_mlstm's; without a workspace heads of 128 x 128 take the kernel
+ * for all other sizes, which waits for nothing.
  */
 typedef struct dz_lightning_args {
   const void* x;

@@ -101,3 +101,42 @@ def test_results_do_not_depend_on_when_tiles_arrive(kind):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for other in busy for a, b in zip(quiet, other))
     assert ops.read_status() == 0
+
+
+def test_status_word_of_a_workspace():
+    """A word that a kernel left is read from the first word of the workspace, also after a larger one took its place; a
+    call without room for it takes the kernel that waits for nothing, or is refused where a workspace is asked for."""
+    import ctypes
+    from deltazip_b200 import _lib, ops
+    L = _lib.lib()
+    assert L.dz_lightning_workspace_bytes(200, 1, 2, 128, 1) >= 4
+    assert L.dz_mlstm_workspace_bytes(3, 2) >= 4 + 3 * 2 * 4
+    assert ops.read_status() == 0
+    a = MlstmRun(2, 128, 128, 140, BF16, seed=3)
+    a.run([140])
+    ops._zeroed_scratch("mlstm", a.x.device, 4)[:4].view(torch.int32).fill_(_lib.DZ_ERR_TIMEOUT)
+    many = 4096                                    # more (sequence, head) pairs than the workspace has room for
+    starts = torch.zeros(many + 1, dtype=torch.int32, device="cuda")
+    ops.mlstm(a.x, a.h, a.w, a.b, a.norm, a.S, a.n, a.m, i32([0] * many), starts, i32([0] * many), a.cap, a.scale, a.eps, True)
+    assert ops.read_status() == _lib.DZ_ERR_TIMEOUT and ops.read_status() == 0
+
+    b = LightningRun(2, 128, 128, 200, BF16, seed=3)
+    ops._zeroed_scratch("lightning_chunk", b.x.device, 4)[:4].view(torch.int32).fill_(_lib.DZ_ERR_TIMEOUT)
+    assert ops.read_status() == _lib.DZ_ERR_TIMEOUT and ops.read_status() == 0
+    out, S = torch.empty((200, 256), dtype=BF16, device="cuda"), torch.zeros((1, 2, 128, 128), device="cuda")
+    slots, starts, ctx = i32([0]), i32([0, 200]), i32([0])
+    args = _lib.LightningArgs(
+        x=b.x.data_ptr(), row_stride=b.x.stride(0), k_off=256, v_off=512, g_off=768, powers=b.powers.data_ptr(),
+        norm_weight=b.norm.data_ptr(), eps=b.eps, out=out.data_ptr(), S=S.data_ptr(), slots=slots.data_ptr(),
+        q_starts=starts.data_ptr(), ctx_lens=ctx.data_ptr(), num_seqs=1, rows=200, heads=2, dim=128, vdim=128, chunkwise=1,
+        dtype=_lib.DZ_DTYPE_BF16)
+    assert L.dz_lightning(ctypes.byref(args), ops._stream()) == 0
+    assert rel(out.double().cpu().numpy(), b.want) < EXACT[BF16]
+    small = torch.zeros(64, dtype=torch.uint8, device="cuda")
+    x = a.x
+    margs = _lib.MlstmArgs(
+        x=x.data_ptr(), row_stride=x.stride(0), k_off=256, v_off=512, g_off=768, b_if=a.b.data_ptr(), pre_if=S.data_ptr(), width=48,
+        cap=a.cap, scale=a.scale, norm_weight=a.norm.data_ptr(), eps=a.eps, out=out.data_ptr(), S=a.S.data_ptr(), n=a.n.data_ptr(),
+        m=a.m.data_ptr(), slots=slots.data_ptr(), q_starts=starts.data_ptr(), ctx_lens=ctx.data_ptr(), num_seqs=1, rows=140,
+        heads=2, dim=128, vdim=128, chunkwise=1, workspace=small.data_ptr(), workspace_bytes=64, dtype=_lib.DZ_DTYPE_BF16)
+    assert L.dz_mlstm(ctypes.byref(margs), ops._stream()) == _lib.DZ_ERR_WORKSPACE
