@@ -202,7 +202,7 @@ paged_decode_attention_kernel(const T* __restrict__ qkv, int q_row_stride, T* __
   // counts is bytes in flight.  A half-warp owns a row (16 lanes x 16 bytes), a warp two rows
   // per load instruction, and two such pairs are requested per iteration: 64 bytes in flight
   // per lane.  Each half-warp keeps its own running (max, sum, accumulator); the halves are
-  // merged by shuffles at the end, the warps through shared memory as in the general form.
+  // merged by shuffles at the end, the warps through shared memory.
   const int half = lane >> 4, hl = lane & 15;
   float q[G][8];
 #pragma unroll
