@@ -617,7 +617,7 @@ def paged_attention_decode(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: to
     if out is None:
         out = torch.empty((b, q_heads * 128), dtype=qkv.dtype, device=qkv.device)
     ws_ptr, ws_bytes = None, 0
-    if q_heads // kv_heads > 2:
+    if splits >= 1 and kv_heads > 0 and q_heads // kv_heads > 2:      # (what the library refuses it is to see)
         splits = _grouped_splits(b, q_heads, kv_heads, block_tables.shape[1] * block_size, splits)
     if splits > 1:
         need = lib().dz_paged_attention_workspace_bytes(b, q_heads, kv_heads, splits)

@@ -174,3 +174,13 @@ def test_infinities_among_the_values(length, key, dtype):
     bad = torch.isinf(want)
     assert torch.equal(torch.where(bad, out[0].double(), 0), torch.where(bad, want, 0)) and int(bad.sum()) == 2 * heads
     check(out[0][~bad], want[~bad], dtype)
+
+
+@pytest.mark.parametrize("heads", [2, 8])
+@pytest.mark.parametrize("splits", [0, -1, 65])
+def test_split_counts_out_of_range_are_refused(heads, splits):
+    from deltazip_b200 import ops
+    from deltazip_b200._lib import DeltaZipError
+    qkv, k, v, tables = batch(1, heads, torch.float16, 1, 40, [600])
+    with pytest.raises(DeltaZipError):
+        ops.paged_attention_decode(qkv, k, v, tables, torch.tensor([600], dtype=torch.int32, device="cuda"), heads, 1, BLOCK, 0.1, splits)
