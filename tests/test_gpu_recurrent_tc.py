@@ -140,3 +140,23 @@ def test_status_word_of_a_workspace():
         m=a.m.data_ptr(), slots=slots.data_ptr(), q_starts=starts.data_ptr(), ctx_lens=ctx.data_ptr(), num_seqs=1, rows=140,
         heads=2, dim=128, vdim=128, chunkwise=1, workspace=small.data_ptr(), workspace_bytes=64, dtype=_lib.DZ_DTYPE_BF16)
     assert L.dz_mlstm(ctypes.byref(margs), ops._stream()) == _lib.DZ_ERR_WORKSPACE
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_silu_far_below_zero_and_next_to_a_nan(dim):
+    """SiLU of -50 is -1e-20, which bf16 holds; a NaN stays in its own column of the state."""
+    from deltazip_b200 import ops
+    r = LightningRun(1, dim, dim, 70, BF16, seed=8, decay=[0.9])
+    x = r.x[:, :4 * dim].clone()
+    x[:, 2 * dim + 3] = -50
+    S = torch.zeros((1, 1, dim, dim), device="cuda")
+    ops.lightning(x, r.powers, r.norm, S, i32([0]), i32([0, 70]), i32([0]), r.eps, True)
+    silu = lambda t: torch.nn.functional.silu(t.double()).to(BF16).double()
+    decay = 0.9 ** torch.arange(69, -1, -1, device="cuda", dtype=torch.float64)
+    want = (silu(x[:, dim:2 * dim]) * decay[:, None]).t() @ silu(x[:, 2 * dim:3 * dim])
+    err = (S[0, 0].double() - want).norm(dim=0) / want.norm(dim=0)          # a column of the state per component of v
+    assert float(err.max()) < 1e-2 and float(S[0, 0, :, 3].abs().max()) > 0
+    x[9, 2 * dim + 5] = float("nan")
+    S.zero_()
+    ops.lightning(x, r.powers, r.norm, S, i32([0]), i32([0, 70]), i32([0]), r.eps, True)
+    assert torch.isnan(S[0, 0]).any(0).nonzero().flatten().tolist() == [5]
