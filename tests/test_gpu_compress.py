@@ -116,3 +116,40 @@ def test_full_size_layer_compresses_and_serves():
     y = ops.apply_delta(xs, qs, ss, ms, idx, w).float()
     ref = xs.float() @ (w.float() + dense).t()
     assert ((y - ref).norm() / ref.norm()).item() <= 2e-3
+
+
+def _columns_one_by_one(delta, hinv, scale, zero, bits):
+    """Pruning, quantisation and error feedback column by column in 64 bits, every column's error fed to all behind it."""
+    W, U = delta.double(), hinv.double()
+    sc, zp = scale.double(), zero.double()
+    out, loss = torch.zeros_like(W), 0.0
+    for i in range(W.shape[1]):
+        d = U[i, i]
+        if i % 4 == 0:
+            importance = W[:, i:i + 4].square() / U.diag()[i:i + 4].square()
+            low = torch.zeros_like(importance, dtype=torch.bool).scatter_(1, importance.sort(dim=1, stable=True).indices[:, :2], True)
+        w = W[:, i].clone()
+        kept = torch.where(low[:, i % 4], 0, w)
+        out[:, i] = sc * ((kept / sc).round().add(zp).clamp(0, 2 ** bits - 1) - zp)
+        err = (w - out[:, i]) / d
+        loss += 0.5 * float(err.square().sum())
+        W[:, i:] -= err[:, None] * U[i, i:]
+    return out, loss
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("k", [512, 516, 640, 1100])
+def test_error_feedback_across_spans_of_blocks(k, bits):
+    """Columns behind a span of four blocks are updated once for the span, those within it per block.  A decision that
+    rounding turns (a weight within 2^-24 x K of a boundary: fewer than one row here) changes the rest of its row: at most
+    two of 64 rows may differ; a block without its update changes them all."""
+    from deltazip_b200 import compress
+    g = torch.Generator(device="cuda").manual_seed(k)
+    delta = torch.randn((64, k), generator=g, device="cuda") * 1e-3
+    x = torch.randn((k // 2, k), generator=g, device="cuda") * (0.25 + 2 * torch.rand(k, generator=g, device="cuda"))
+    hinv, _ = compress.hinv_factor(x.t() @ x, 0.05)
+    got, scale, zero, loss = compress.sparsegpt_2_4(delta, bits, hinv=hinv)
+    want, total = _columns_one_by_one(delta, hinv, scale, zero, bits)
+    differ = (got.double() - want).abs() > scale.double()[:, None] * 0.5
+    assert int(differ.any(1).sum()) <= 2, differ.any(1).sum()
+    assert abs(loss.double().sum().item() - total) <= 1e-3 * total
