@@ -6,10 +6,11 @@
 // are four products per chunk, 56 MMAs of 128 x 128 x 16.  The state, P and w V, held in 32 bits, enter them as hi +
 // lo pairs of the 16-bit type; the state itself stays in 32 bits in registers.
 //
-// Bound by the sixteen warps: of 10 to 13 thousand cycles a chunk SiLU takes 5 (lightning; the special function unit),
-// the exponentials and sums of the gates 4 and the output gate 5 (matrix memory), the products wait for them.
+// Bound by the sixteen warps: of about 17 thousand cycles a chunk (one warp's clock, 1965 MHz) SiLU takes 8.7 (constant
+// decay; the special function unit); in the matrix memory w V and the sums for n and q.n take 3, the weights of P and the
+// scaling of O 3, the output with its norm and gate 9.  Waits for the products come to 0.4 and 0.9.
 // Measured against the warp-MMA kernels of 64 tokens at a time, bf16: matrix memory, 4 prompts of up to 2048 tokens x
-// 32 heads, 566 -> 170 us; constant decay, 5 prompts of up to 1500 x 16 heads, continued, 260 -> 133 us.
+// 32 heads, 565 -> 170 us; constant decay, 5 prompts of up to 1500 x 16 heads, continued, 260 -> 135 us.
 //
 // Tensor memory (128 columns each): scores, then P in their place | O | the update | w V.
 // Shared memory: a ring of four tiles of 128 x 128 (q, k, v, q, ...) and S as the product with q reads it.
@@ -63,6 +64,13 @@ __device__ __forceinline__ void warp_umma_ts(uint32_t d, uint32_t a, uint32_t b_
 __device__ __forceinline__ void cp_async16_u32(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
+struct Sum { float hi, lo; };            // hi + lo, lo below hi's last place
+// (Knuth's two-sum: hi takes the rounded sum, lo what the rounding left.)
+__device__ __forceinline__ Sum add(Sum a, Sum b) {
+  const float s = a.hi + b.hi, t = s - a.hi, lo = ((a.hi - (s - t)) + (b.hi - t)) + (a.lo + b.lo), hi = s + lo;
+  return {hi, lo - (hi - s)};
+}
+__device__ __forceinline__ float apart(Sum a, Sum b) { return (a.hi - b.hi) + (a.lo - b.lo); }
 template <typename T> __device__ __forceinline__ float lds_one(uint32_t a) {
   unsigned short v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
               const int s = c0 + g * 16 + 2 * j + e;
               float w;
               if constexpr (MEMORY) {
-                w = ex2((cw.a[s] - own) * kLog2e) * p.scale;
+                w = __expf(cw.a[s] - own) * p.scale;
                 w = s <= r ? w : 0.f;
               } else {
                 w = s_pw[kTok + r - s];
@@ -359,8 +367,8 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
             for (int j = 0; j < 4; ++j) {
               const float2 e = Cvt<T>::up(g[j]);
               const int k = c * 8 + 2 * j;
-              f[2 * j] = __fdividef(o[k] * rms * s_nw[c0 + k], 1.f + __expf(-e.x));
-              f[2 * j + 1] = __fdividef(o[k + 1] * rms * s_nw[c0 + k + 1], 1.f + __expf(-e.y));
+              f[2 * j] = o[k] * rms * s_nw[c0 + k] / (1.f + __expf(-e.x));
+              f[2 * j + 1] = o[k + 1] * rms * s_nw[c0 + k + 1] / (1.f + __expf(-e.y));
             }
             store8<T>(op + c * 8, f);
           }
@@ -453,8 +461,8 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
 #pragma unroll
       for (int j = 0; j < 8; ++j) {                      // 16 tokens: 2048 bytes of a tile
         const uint32_t a = tmem + kTW + (j >> 1) * 32 + (j & 1) * 8;
-        warp_umma_ts(tmem + kTU, a, dkm + j * 128, id_mn, j > 0);
-        warp_umma_ts(tmem + kTU, a + 16, dkm + j * 128, id_mn, 1);
+        warp_umma_ts(tmem + kTU, a + 16, dkm + j * 128, id_mn, j > 0);      // lo while the sums are smaller
+        warp_umma_ts(tmem + kTU, a, dkm + j * 128, id_mn, 1);
       }
       warp_umma_commit(smem_u32(&b_u));
       warp_umma_commit(smem_u32(&b_empty[nk & 3]));
@@ -472,36 +480,38 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
       warp_umma_commit(smem_u32(&b_empty[nv & 3]));
     }
   } else if constexpr (MEMORY) {
-    // ---- the chunk's weights; a lane holds four tokens ----
-    float m = ctx > 0 ? p.m[(size_t)slot * p.heads + head] : 0.f;
+    // ---- the chunk's weights; a lane holds four tokens.  A sum of 128 gates is kept as hi + lo, weights are taken
+    // against the chunk's last maximum: what a weight's logarithm is off by does not grow with the sums ----
+    Sum m = {ctx > 0 ? p.m[(size_t)slot * p.heads + head] : 0.f, 0.f};
     for (int i = 0; i < chunks; ++i) {
       const int base = i * kTok, len = min(kTok, qn - base), t = 4 * lane;
       ChunkWeights& cw = s_cw[i & 1];
-      float gi[4], F[4], M[4];
+      Sum F[4], a[4];
+      float gi[4], M[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         gi[j] = -INFINITY;                               // absent tokens add nothing and forget nothing
-        F[j] = 0.f;
+        F[j] = {0.f, 0.f};
         if (t + j < len) {
           const float* pre = p.pre_if + (size_t)(q0 + base + t + j) * 2 * p.heads + head;
           gi[j] = soft_cap(pre[0] + p.b_if[head], p.cap);
-          F[j] = log_sigmoid(soft_cap(pre[p.heads] + p.b_if[p.heads + head], p.cap));
+          F[j].hi = log_sigmoid(soft_cap(pre[p.heads] + p.b_if[p.heads + head], p.cap));
         }
       }
 #pragma unroll
-      for (int j = 1; j < 4; ++j) F[j] += F[j - 1];
-      float sum = F[3];
+      for (int j = 1; j < 4; ++j) F[j] = add(F[j], F[j - 1]);
+      Sum sum = F[3];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, sum, o);
-        if (lane >= o) sum += up;
+        const Sum up = {__shfl_up_sync(0xffffffffu, sum.hi, o), __shfl_up_sync(0xffffffffu, sum.lo, o)};
+        if (lane >= o) sum = add(sum, up);
       }
-      const float before = __shfl_up_sync(0xffffffffu, sum, 1);
+      const Sum before = {__shfl_up_sync(0xffffffffu, sum.hi, 1), __shfl_up_sync(0xffffffffu, sum.lo, 1)};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (lane > 0) F[j] += before;
-        gi[j] -= F[j];
-        M[j] = j > 0 ? fmaxf(M[j - 1], gi[j]) : gi[j];
+        if (lane > 0) F[j] = add(F[j], before);
+        a[j] = t + j < len ? add({gi[j], 0.f}, {-F[j].hi, -F[j].lo}) : Sum{-INFINITY, 0.f};
+        M[j] = j > 0 ? fmaxf(M[j - 1], a[j].hi) : a[j].hi;     // (a row may take any M near its largest)
       }
       float mx = M[3];
 #pragma unroll
@@ -510,24 +520,32 @@ __global__ void __launch_bounds__(kThreadsRec, 1) recurrent_chunk_tc_kernel(cons
         if (lane >= o) mx = fmaxf(mx, up);
       }
       float top = __shfl_up_sync(0xffffffffu, mx, 1);
-      top = lane > 0 ? fmaxf(top, m) : m;
+      top = lane > 0 ? fmaxf(top, m.hi) : m.hi;
 #pragma unroll
       for (int j = 0; j < 4; ++j) M[j] = fmaxf(M[j], top);
-      const float ML = __shfl_sync(0xffffffffu, M[3], 31), FL = __shfl_sync(0xffffffffu, F[3], 31);
+      // the last one goes into m: with the lo of whose hi it is
+      Sum ML = {__shfl_sync(0xffffffffu, M[3], 31), 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ML.lo = a[j].hi == ML.hi ? a[j].lo : ML.lo;
+      const unsigned holders = __ballot_sync(0xffffffffu, a[0].hi == ML.hi || a[1].hi == ML.hi || a[2].hi == ML.hi || a[3].hi == ML.hi);
+      ML.lo = __shfl_sync(0xffffffffu, ML.lo, holders ? __ffs(holders) - 1 : 0);
+      if (!holders) ML.lo = m.lo;
+      const Sum FL = {__shfl_sync(0xffffffffu, F[3].hi, 31), __shfl_sync(0xffffffffu, F[3].lo, 31)};
       bar_wait(&b_wempty[i & 1], ((i >> 1) & 1) ^ 1, abort_flag, p.status);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        cw.a[t + j] = gi[j];
-        cw.mx[t + j] = M[j];
-        cw.in[t + j] = expf(m - M[j]) * p.scale;
-        cw.em[t + j] = expf(-(F[j] + M[j]));
-        cw.w[t + j] = expf(gi[j] - ML);
+        const float rel = apart(a[j], ML);
+        cw.a[t + j] = rel;
+        cw.mx[t + j] = (M[j] - ML.hi) - ML.lo;
+        cw.in[t + j] = expf((m.hi - M[j]) + m.lo) * p.scale;
+        cw.em[t + j] = expf(-((F[j].hi + M[j]) + F[j].lo));
+        cw.w[t + j] = expf(rel);
       }
-      if (lane == 0) cw.decay = expf(m - ML);
-      m = FL + ML;
+      if (lane == 0) cw.decay = expf(apart(m, ML));
+      m = add(FL, ML);
       mbar_arrive(smem_u32(&b_wfull[i & 1]));
     }
-    if (lane == 0) p.m[(size_t)slot * p.heads + head] = m;
+    if (lane == 0) p.m[(size_t)slot * p.heads + head] = m.hi;
   }
 
   tc_fence_before();

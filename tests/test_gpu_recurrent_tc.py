@@ -160,3 +160,27 @@ def test_silu_far_below_zero_and_next_to_a_nan(dim):
     S.zero_()
     ops.lightning(x, r.powers, r.norm, S, i32([0]), i32([0, 70]), i32([0]), r.eps, True)
     assert torch.isnan(S[0, 0]).any(0).nonzero().flatten().tolist() == [5]
+
+
+def test_gate_sums_of_a_chunk_keep_their_precision():
+    """Forget gates near 0.1: the logarithms of a chunk add up to -300, whose last place is 3e-5.  What a weight's logarithm
+    may be off by is the roundings of a gate of size 3 (cap, tanh, logarithm: 2^-22 each) for the few tokens that count;
+    the gates' inputs are exact in 32 bits.  The bound is 2^-19."""
+    from deltazip_b200 import ops
+    t, heads = 600, 2
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn((t, heads * 512), generator=g, device="cuda").to(BF16)
+    h = torch.randint(-3, 4, (t, 16), generator=g, device="cuda").to(BF16)
+    w = (torch.randint(-1, 2, (2 * heads, 16), generator=g, device="cuda") / 8).to(BF16)
+    b = torch.tensor([0.5, -1.0, -2.25, -2.5], device="cuda")
+    S, n, m = (torch.zeros(s, device="cuda") for s in ((1, heads, 128, 128), (1, heads, 128), (1, heads)))
+    ops.mlstm(x, h, w, b, torch.ones(heads * 128, device="cuda"), S, n, m, i32([0]), i32([0, t]), i32([0]), 64.0, 0.1, 1e-6, True)
+    pre = 64 * torch.tanh((h.double() @ w.double().t() + b.double()) / 64)
+    i, F = pre[:, :heads].t(), torch.nn.functional.logsigmoid(pre[:, heads:]).t().cumsum(1)
+    top = torch.maximum((i - F).cummax(1).values, torch.zeros((), device="cuda", dtype=torch.float64))[:, -1:]
+    last = (i - F - top).exp()
+    k = x[:, heads * 128:heads * 256].double().view(t, heads, 128)
+    want = torch.einsum("ht,thd->hd", last, k)
+    assert float(F.min()) < -1000
+    assert float((n[0].double() - want).norm() / want.norm()) <= 2.0 ** -19
+    assert float((m[0].double() - (F[:, -1:] + top)[:, 0]).abs().max()) <= 2.0 ** -19
