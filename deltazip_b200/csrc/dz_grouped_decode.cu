@@ -58,7 +58,12 @@ grouped_decode_kernel(GroupedDecode p) {
   pdl_wait();
   pdl_launch();
   const int len = p.lens[seq] + p.more, lo = p.window > 0 ? max(0, len - p.window) : 0;
-  const int per = ((len - lo + p.splits - 1) / p.splits + kTile - 1) / kTile * kTile;
+  // A step of the CTA takes a tile for each of its warps: no split has fewer keys, and those left without any end here.
+  // (The count may come from the table's width, of which a short sequence fills little.)
+  constexpr int kStep = kWarps * kTile;
+  const int per = max(((len - lo + p.splits - 1) / p.splits + kTile - 1) / kTile * kTile, kStep);
+  const int splits = max(1, (len - lo + per - 1) / per);
+  if (split >= splits) return;
   const int t0 = lo + split * per, t1 = min(len, t0 + per);
   const int* table = p.tables + (size_t)seq * p.ring_blocks;
   const T* kc = (const T*)p.k_cache;
@@ -227,7 +232,7 @@ grouped_decode_kernel(GroupedDecode p) {
       a[2] += v.z * c;
       a[3] += v.w * c;
     }
-    if (p.splits == 1) {
+    if (splits == 1) {
       store(h, d, a, sum);
     } else {
       const size_t at = (column + h) * p.splits + split;
@@ -235,13 +240,13 @@ grouped_decode_kernel(GroupedDecode p) {
       if (d == 0) ml[at] = make_float2(mm, sum);
     }
   }
-  if (p.splits == 1) return;
+  if (splits == 1) return;
   // the last split of this column to finish merges all of them; nothing waits
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     int* ticket = p.tickets + (size_t)seq * gridDim.x + blockIdx.x;
-    s_last = atomicAdd(ticket, 1) == p.splits - 1;
+    s_last = atomicAdd(ticket, 1) == splits - 1;
     if (s_last) *ticket = 0;                                   // ready for the next launch
   }
   __syncthreads();
@@ -251,9 +256,9 @@ grouped_decode_kernel(GroupedDecode p) {
     const int h = i / kGroupedDim, d = i % kGroupedDim;
     const size_t at = (column + h) * p.splits;
     float mm = -INFINITY, sum = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, __ldcg(&ml[at + s]).x);
+    for (int s = 0; s < splits; ++s) mm = fmaxf(mm, __ldcg(&ml[at + s]).x);
 #pragma unroll 4
-    for (int s = 0; s < p.splits; ++s) {
+    for (int s = 0; s < splits; ++s) {
       const float2 w = __ldcg(&ml[at + s]);
       const float4 v = __ldcg(reinterpret_cast<const float4*>(p.partial + (at + s) * kGroupedDim + d));
       const float c = w.x == -INFINITY ? 0.f : __expf(w.x - mm);

@@ -184,3 +184,22 @@ def test_split_counts_out_of_range_are_refused(heads, splits):
     qkv, k, v, tables = batch(1, heads, torch.float16, 1, 40, [600])
     with pytest.raises(DeltaZipError):
         ops.paged_attention_decode(qkv, k, v, tables, torch.tensor([600], dtype=torch.int32, device="cuda"), heads, 1, BLOCK, 0.1, splits)
+
+
+@pytest.mark.parametrize("heads,kvh", [(8, 1), (32, 8)])
+def test_short_sequences_in_wide_tables(heads, kvh):
+    """The number of splits follows from the tables' width; splits that a sequence has no keys for take no part, in the
+    merge and in the tickets."""
+    from deltazip_b200 import ops
+    dtype, lens = torch.float16, [1, 64, 65, 300, 1000, 0]
+    qkv, k, v, tables = batch(kvh, heads, dtype, 9, 256, lens)
+    for rep in range(3):
+        order = list(range(len(lens)))[::-1] if rep == 1 else list(range(len(lens)))     # the tickets are back at zero
+        n = torch.tensor([lens[i] for i in order], dtype=torch.int32, device="cuda")
+        out = ops.paged_attention_decode(qkv, k, v, tables, n, heads, kvh, BLOCK, 128 ** -0.5)
+        for row, i in enumerate(order):
+            at = (tables[row].long()[:, None] * BLOCK + torch.arange(BLOCK, device="cuda")).flatten()[:lens[i]]
+            if lens[i] == 0:
+                assert not out[row].any()
+            else:
+                check(out[row], reference(qkv[row, :heads * 128].view(heads, 128), k[at], v[at], 128 ** -0.5), dtype)
