@@ -29,12 +29,8 @@ from ._lib import SbmmArgs, check, lib
 
 # Largest batch (rows of x) that takes the fused kernel for base and delta products together.
 FUSED_MAX_TOKENS = 512
-# The delta products of such a batch are added by the prompt kernel, but for two cases of a sorted batch whose runs are
-# known on the host (Segments.host_runs) and have DENSE_RUN_TOKENS rows or more: there a slot is dequantised (dz_unpack)
-# and multiplied by the library GEMM, as the reference's PyTorch path does (deltazip/nn_modules/qlinear.py:266-330).
-# One is a single slot's rows over a matrix of at most DENSE_RUN_SIZE entries, too small to give every SM a tile (1280 x
-# 2048, 2048 rows: dequantised 38 us, prompt kernel 48; 4096 x 4096: 126 and 122; three slots of 1280 x 2048: 100 and
-# 48), the other a stack of more slots than the prompt kernel has tables for.
+# The delta products of such a batch are added by the prompt kernel, but for some sorted batches whose runs are known on the
+# host (Segments.host_runs) and have DENSE_RUN_TOKENS rows or more (_dequantise_runs).
 PREFILL_MAX_SLOTS = 1024
 DENSE_RUN_SIZE = 1 << 23
 DENSE_RUN_TOKENS = 256
@@ -131,7 +127,7 @@ class Segments:
         self.m = 0
         self.sorted = False
         # [(slot, first row, end row)] of a sorted batch when the caller knows it on the host
-        # (the slot manager does); None otherwise.  Only prefill-sized batches over very many slots use it.
+        # (the slot manager does); None otherwise.  Decides how prefill-sized batches are multiplied (_dequantise_runs).
         self.host_runs = None
 
     def build(self, indices: torch.Tensor, sorted_hint: Optional[bool] = None) -> "Segments":
@@ -219,6 +215,31 @@ def _bits_from_shapes(qweight_stacked: torch.Tensor, k: int) -> int:
     return qweight_stacked.shape[-2] * 128 // k
 
 
+def _dequantise_runs(n: int, k: int, slots: int, runs) -> bool:
+    """Whether the slots of a prompt batch are dequantised one after the other (dz_unpack) and multiplied by the library
+    GEMM, as the reference's PyTorch path does (deltazip/nn_modules/qlinear.py:266-330), in place of the prompt kernel.
+
+    The kernel wants a tile for every SM and many steps over k for the pass over y that ends a tile; dequantising costs a
+    pass over the matrix, and 18 us of the host, for each slot.  Times of the whole call on the device, kernel and
+    dequantised, 4-bit, in us:
+    one slot, a small matrix (4096 x 1024, 2048 rows: 50 and 37; 4096 x 2048: 69 and 61; 5632 x 2048: 80 and 83);
+    one slot, few steps over k (16384 x 512: 114 and 87; 11008 x 1024, 2048 rows: 102 and 93, 600 rows: 43 and 38, which is
+    the host's time; 13824 x 1280: 128 and 127, 13824 x 1536: 140 and 151);
+    one slot, few tiles (1024 x 11008, 600 rows: 93 and 51, 3000 rows: 113 and 111; 2048 x 11008, 1024 rows: 95 and 93, 2048
+    rows: 125 and 149);
+    two or three slots, very few steps and a y that outweighs the host's time (16384 x 512, 2048 rows of three: 117 and 107,
+    of six: 119 and 139; 4096 x 1024, 2048 rows of two: 49 and 43, behind 64 of the host's)."""
+    lengths = [end - start for slot, start, end in runs if slot >= 0]
+    if any(length < DENSE_RUN_TOKENS for length in lengths):
+        return False
+    if slots > PREFILL_MAX_SLOTS:                  # the kernel has no tables for them
+        return True
+    rows = sum(lengths)
+    if len(lengths) == 1:
+        return n * k <= DENSE_RUN_SIZE or k <= 512 or (k <= 1280 and rows >= 1024) or (n <= 2048 and n * rows < 1 << 22)
+    return len(lengths) <= 3 and k <= 512 and n * rows >= 1 << 25
+
+
 def sbmm(x: torch.Tensor, qweight_stacked: torch.Tensor, scales_stacked: torch.Tensor,
          meta_stacked: torch.Tensor, segments: Segments, base_weight: Optional[torch.Tensor],
          out: Optional[torch.Tensor] = None, bits: Optional[int] = None,
@@ -265,10 +286,7 @@ def sbmm(x: torch.Tensor, qweight_stacked: torch.Tensor, scales_stacked: torch.T
             else:
                 o2.copy_(base)
         runs = segments.host_runs
-        if runs is not None and segments.sorted and \
-                (qweight_stacked.shape[0] > PREFILL_MAX_SLOTS or
-                 (n * k <= DENSE_RUN_SIZE and sum(slot >= 0 for slot, _, _ in runs) == 1)) and \
-                all(e - s >= DENSE_RUN_TOKENS for slot, s, e in runs if slot >= 0):
+        if runs is not None and segments.sorted and _dequantise_runs(n, k, qweight_stacked.shape[0], runs):
             o2 = out.reshape(-1, out.shape[-1]) if out.dim() != 2 else out
             for slot, s, e in runs:
                 if slot < 0:

@@ -299,38 +299,57 @@ def test_prefill_sized_batch_takes_the_split_path_and_agrees_with_the_fused_one(
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("bits", [2, 4])
-def test_prefill_runs_known_on_the_host_take_the_dequantise_once_path(bits):
+@pytest.mark.parametrize("n,k,slots,lens,size,dequantised", [
+    (2176, 1536, 3, [(-1, 300), (0, 600)], 2176 * 1536, 1),          # one delta, a matrix just small enough
+    (2176, 1536, 3, [(-1, 300), (0, 256)], 2176 * 1536, 1),          # the shortest run that counts as long
+    (2176, 1536, 3, [(-1, 300), (0, 600)], 2176 * 1536 - 1, 0),      # just too large
+    (2176, 1536, 3, [(-1, 400), (0, 255)], 2176 * 1536, 0),          # a run too short
+    (2176, 1536, 3, [(-1, 300), (0, 600), (2, 400)], 2176 * 1536, 0),            # two deltas
+    (2176, 512, 3, [(0, 600)], 0, 1), (2176, 576, 3, [(0, 600)], 0, 0),          # few steps over k
+    (2176, 1280, 3, [(-1, 5), (1, 1024)], 0, 1), (2176, 1280, 3, [(-1, 5), (1, 1023)], 0, 0),
+    (2048, 1536, 3, [(1, 2047)], 0, 1), (2048, 1536, 3, [(1, 2048)], 0, 0),      # few tiles
+    (16384, 512, 4, [(0, 1024), (1, 1024)], 0, 2), (16384, 512, 4, [(0, 1024), (1, 1023)], 0, 0),
+    (16384, 512, 4, [(0, 512), (1, 512), (2, 512), (3, 512)], 0, 0),
+    (128, 64, 1025, [(-1, 10), (0, 300), (7, 256), (1024, 400)], 0, 3),          # more slots than the prompt kernel takes
+    (128, 64, 1025, [(-1, 10), (0, 300), (7, 255), (1024, 400)], 0, 0),          # ... and a run too short
+    (128, 64, 1024, [(-1, 10), (0, 300), (7, 256), (1023, 400)], 0, 0)])         # as many as it takes
+def test_prefill_runs_known_on_the_host_and_the_dequantise_once_path(monkeypatch, n, k, slots, lens, size, dequantised, bits):
     """A sorted prefill-sized batch whose runs the caller knows (Segments.host_runs, as the slot
-    manager provides) multiplies each long run by the slot's dequantised delta through the
-    library GEMM; the result must agree with the kernel path and with the fp32 reference."""
+    manager provides): which runs are multiplied by the slot's dequantised delta through the library
+    GEMM, and that the result agrees with that of the kernels (taken where the runs are not known)
+    and with the fp32 reference."""
     from deltazip_b200 import ops, synth
     dev = torch.device("cuda")
-    n, k, slots = 1024, 1024, 3
-    lens = [300, 600, 256, 400]                      # base rows, slot 0, slot 1, slot 2
-    idx = torch.cat([torch.full((c,), s - 1, dtype=torch.int64) for s, c in enumerate(lens)]).to(dev)
+    monkeypatch.setattr(ops, "DENSE_RUN_SIZE", size)
+    idx = torch.cat([torch.full((c,), s, dtype=torch.int64) for s, c in lens]).to(dev)
     m = idx.numel()
     g = torch.Generator(device=dev).manual_seed(11)
     w = (torch.randn((n, k), generator=g, device=dev) * 0.02).half()
     x = torch.randn((m, k), generator=g, device=dev).half()
     qw, meta, sc = synth.random_delta_slots(slots, n, k, bits, seed=5, device=dev, std=1e-2)
+    want, at, runs = x.float() @ w.float().t(), 0, []
+    for s, c in lens:
+        if s >= 0:
+            want[at:at + c] += x[at:at + c].float() @ ops.unpack(qw[s], meta[s], sc[s], n, k, bits).float().t()
+        runs.append((s, at, at + c))
+        at += c
+    calls, unpack = [], ops.unpack
+    monkeypatch.setattr(ops, "unpack", lambda *a, **kw: calls.append(a) or unpack(*a, **kw))
     seg = ops.Segments(m, slots, dev).build(idx, sorted_hint=True)
     kernel_path = ops.sbmm(x, qw, sc, meta, seg, w)
-    edges = [0]
-    for c in lens:
-        edges.append(edges[-1] + c)
-    seg.host_runs = [(s - 1, edges[s], edges[s + 1]) for s in range(len(lens))]
-    dense_path = ops.sbmm(x, qw, sc, meta, seg, w)
-    want = x.float() @ w.float().t()
-    for s in range(slots):
-        rows = (idx == s).nonzero().flatten()
-        want[rows] += x[rows].float() @ ops.unpack(qw[s], meta[s], sc[s], n, k, bits).float().t()
-    assert ((dense_path.float() - want).norm() / want.norm()).item() <= 2e-3
-    assert ((dense_path.float() - kernel_path.float()).norm() / want.norm()).item() <= 2e-3
-    # a short run sends the whole call back to the kernel
-    seg.host_runs = [(-1, 0, 300), (0, 300, 900), (1, 900, 1000), (1, 1000, 1156), (2, 1156, m)]
-    again = ops.sbmm(x, qw, sc, meta, seg, w)
-    assert torch.equal(again, kernel_path)
-    # the slot manager's mapping yields the runs for such a batch
+    assert not calls
+    seg.host_runs = runs
+    got = ops.sbmm(x, qw, sc, meta, seg, w)
+    assert len(calls) == dequantised
+    if not dequantised:
+        assert torch.equal(got, kernel_path)
+    for y in (got, kernel_path):
+        assert ((y.float() - want).norm() / want.norm()).item() <= 2e-3
+    assert ops.read_status(dev) == 0
+
+
+def test_the_slot_manager_yields_the_runs_of_a_prefill_batch():
+    dev = torch.device("cuda")
     from deltazip_b200.models import DeltaMapping, _convert_mapping
     ids = [0] * 300 + [7] * 600 + [9] * 700
     _, (is_sorted, runs) = _convert_mapping(DeltaMapping(ids, [0, 7, 9]), [7, 9, None], 4, 32000, 0, device=dev)
