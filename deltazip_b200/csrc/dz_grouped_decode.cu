@@ -59,7 +59,8 @@ grouped_decode_kernel(GroupedDecode p) {
   pdl_launch();
   const int len = p.lens[seq] + p.more, lo = p.window > 0 ? max(0, len - p.window) : 0;
   // A step of the CTA takes a tile for each of its warps: no split has fewer keys, and those left without any end here.
-  // (The count may come from the table's width, of which a short sequence fills little.)
+  // (The count may come from the table's width, of which a short sequence fills little: 8 heads on 1, 300 keys in a table
+  // for 16384, 25.5 us with every split merged, 7.6 so.)
   constexpr int kStep = kWarps * kTile;
   const int per = max(((len - lo + p.splits - 1) / p.splits + kTile - 1) / kTile * kTile, kStep);
   const int splits = max(1, (len - lo + per - 1) / per);
