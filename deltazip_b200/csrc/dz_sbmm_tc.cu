@@ -110,6 +110,7 @@ constexpr int kWinBytes = 2 * kMaxWindowCols * 128;   // window buffer (B operan
 constexpr int kMaxW = 4, kMaxX = 4, kMaxR = 24, kMaxBuf = 8;
 constexpr int kMaxWin = 128;                   // windows of one token block
 constexpr int kTmemCols = 512;
+constexpr int kNarrowCols = 16;                // token blocks of the narrow form
 constexpr int kSmemBudget = 216 * 1024;
 constexpr int kEpilogueUnits = 2;               // cost of a tile's epilogue in k-units (work split)
 constexpr int kPrefetchTiles = 8;               // W half-tiles prefetched to L2 in the prologue
@@ -224,7 +225,7 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  constexpr bool WIDE = COLS > 64, narrow = COLS <= 16;
+  constexpr bool WIDE = COLS > 64, narrow = COLS <= kNarrowCols;
   constexpr int C = mode_classes(WIDE);
   constexpr int kDcols = mode_dcols(WIDE);
   constexpr int kWStages = mode_w_stages(WIDE), kXStages = mode_x_stages(WIDE);
@@ -449,8 +450,18 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   }
   if ((int)threadIdx.x < kTokenBlock) {
-    s_slot[threadIdx.x] = t_slot;
-    s_tok[threadIdx.x] = t_tok;
+    // Windows of a block of 16 columns are the whole block, and a row belongs to one by its slot: a batch that is no
+    // larger stays in its own order, column c is its row c wherever the table's order has it, and no gather of x runs in
+    // front.  (Above 16 a window is a span of the sorted order.)
+    int c = threadIdx.x;
+    if (narrow && p.M <= kNarrowCols && !bad && c < p.M) {
+      c = t_tok;
+      t_tok = c;
+    }
+    if ((unsigned)c < (unsigned)kTokenBlock) {
+      s_slot[c] = t_slot;
+      s_tok[c] = t_tok;
+    }
   }
   if (threadIdx.x == 0) {
     // freed by the base issuer's commit and, when there are windows, by every thread of every
@@ -669,6 +680,7 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     bool cta_first_fragment = true;
     long long a_x = 0, a_r = 0, a_free = 0, a_exp = 0, a_win = 0, a_fin = 0, a_epi = 0, tq = 0;
     const bool acc_on = INSTR && ep_tid == 0;
+    const int row_slot = narrow ? s_slot[wg_tid >> 3] : 0;   // of the one row this thread copies into a window
 
     for (int u = u_begin; u < u_end;) {
       const int tile = u / KU, ku0 = u % KU;
@@ -736,7 +748,7 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const uint4 zero4 = make_uint4(0, 0, 0, 0);
             for (int c = wg_tid; c < ws.ncols * 8; c += 128) {
               const int row = c >> 3;
-              const bool in = row >= lo && row < hi;
+              const bool in = narrow ? row_slot == ws.slot : row >= lo && row < hi;
               uint4 v0 = zero4, v1 = zero4;
               if (in) {
                 v0 = lds128(x0 + c * 16);
@@ -1078,7 +1090,7 @@ int launch_sbmm(const dz_sbmm_args& a, bool base_only, cudaStream_t st) {
   uint8_t* ws = reinterpret_cast<uint8_t*>(a.workspace);
   const bool sorted = base_only || a.tokens_sorted != 0;
   const void* xsrc = a.x;
-  if (!sorted) {
+  if (!sorted && a.M > kNarrowCols) {     // (the narrow form takes the batch in its own order)
     uint8_t* xs = ws + ((kWsPartials + sbmm_partial_bytes(a.M) + 1023) & ~(size_t)1023);
     gather_rows_kernel<<<a.M, 128, 0, st>>>((const uint4*)a.x, (const uint8_t*)a.segments,
                                              (uint4*)xs, a.M, a.K / 8);
@@ -1168,7 +1180,7 @@ int launch_sbmm(const dz_sbmm_args& a, bool base_only, cudaStream_t st) {
     static const Kern kerns[24] = {DZ_KERNS(false, 16), DZ_KERNS(true, 16), DZ_KERNS(false, 64),
                                    DZ_KERNS(true, 64),  DZ_KERNS(false, 128), DZ_KERNS(true, 128)};
 #undef DZ_KERNS
-    const int kidx = ((a.bits == 2) ? 0 : 1) + (dt ? 2 : 0) + (fullk ? 4 : 0) + (p.cols <= 16 ? 0 : wide ? 16 : 8);
+    const int kidx = ((a.bits == 2) ? 0 : 1) + (dt ? 2 : 0) + (fullk ? 4 : 0) + (p.cols <= kNarrowCols ? 0 : wide ? 16 : 8);
     Kern kern = kerns[kidx];
     if (!di.attr_set[kidx]) {
       DZ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
