@@ -120,23 +120,21 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
     # The columns behind a block are updated up to the end of a span of four blocks, those behind the span once for
     # the whole of it: a quarter of the passes over W, and products four times as deep.
     span = 4 * blocksize
+    errors = torch.empty((n, min(span, k)), dtype=torch.float32, device=W.device)
+    wide = errors.shape[1]
     for s1 in range(0, k, span):
         s2 = min(s1 + span, k)
-        errors = torch.empty((n, s2 - s1), dtype=torch.float32, device=W.device)
         for i1 in range(s1, s2, blocksize):
             i2 = min(i1 + blocksize, s2)
-            count = i2 - i1
-            Q = torch.empty((n, count), dtype=torch.float32, device=W.device)
-            E = torch.empty((n, count), dtype=torch.float32, device=W.device)
-            check(L.dz_sparsegpt_block(W.data_ptr() + 4 * i1, k, hinv.data_ptr() + 4 * (i1 * k + i1), k,
-                                       scale.data_ptr(), zero.data_ptr(), bits, n, count, Q.data_ptr(),
-                                       E.data_ptr(), loss.data_ptr(), _stream()), "dz_sparsegpt_block")
-            W[:, i1:i2] = Q
-            errors[:, i1 - s1:i2 - s1] = E
+            # the quantised block takes the place of the block, its errors theirs in the span's
+            check(L.dz_sparsegpt_block_strided(
+                W.data_ptr() + 4 * i1, k, hinv.data_ptr() + 4 * (i1 * k + i1), k, scale.data_ptr(), zero.data_ptr(), bits,
+                n, i2 - i1, W.data_ptr() + 4 * i1, k, errors.data_ptr() + 4 * (i1 - s1), wide, loss.data_ptr(),
+                _stream()), "dz_sparsegpt_block_strided")
             if i2 < s2:
-                W[:, i2:s2].addmm_(E, hinv[i1:i2, i2:s2], alpha=-1)
+                W[:, i2:s2].addmm_(errors[:, i1 - s1:i2 - s1], hinv[i1:i2, i2:s2], alpha=-1)
         if s2 < k:
-            W[:, s2:].addmm_(errors, hinv[s1:s2, s2:], alpha=-1)
+            W[:, s2:].addmm_(errors[:, :s2 - s1], hinv[s1:s2, s2:], alpha=-1)
     return W, scale, zero, loss
 
 

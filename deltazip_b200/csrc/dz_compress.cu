@@ -8,8 +8,8 @@
 //                            (deltazip/core/quant.py:9-18), and the quantisation / pruning error
 //                            of column i is fed forward into the block's later columns through
 //                            row i of the upper Cholesky factor of H^-1 (:139-141).  Rows of W are
-//                            independent, so one warp owns one row: lane l holds columns l, l+32,
-//                            l+64, l+96 of the block; the block of Hinv sits in shared memory.
+//                            independent; eight lanes own one row, a group of four columns belongs to one lane, and
+//                            the block of Hinv sits in shared memory.
 //                            Outputs Q (quantised block) and Err ((w - q) / Hinv_ii per column),
 //                            from which the caller forms the update of the columns behind the
 //                            block, W[:, i2:] -= Err @ Hinv[i1:i2, i2:] (:146), a plain GEMM.
@@ -29,92 +29,157 @@ namespace {
 
 constexpr int kCBlock = 128;
 
-__device__ __forceinline__ float quantize_sym(float w, float scale, float zero, float maxq) {
-  // quant.py:9-18: q = clamp(round(w / scale) + zero, 0, maxq); return scale * (q - zero)
-  float q = rintf(__fdiv_rn(w, scale)) + zero;
-  q = fminf(fmaxf(q, 0.f), maxq);
-  return __fmul_rn(scale, q - zero);
+// a / b correctly rounded for many a and one b, y = 1 / b correctly rounded: two corrections of a * y by the exact remainder.
+// After the first q is within one unit of the last place, and the second then rounds correctly (Markstein, IBM J. Res. Dev.
+// 34, 1990; Muller et al., Handbook of Floating-Point Arithmetic, 4.7).  That holds while no remainder underflows and
+// nothing overflows: `ok` of the operands, which the caller has to look at before it uses the quotients.  (A zero's sign is
+// not kept.)
+struct Divisor {
+  float b, y;
+};
+__device__ __forceinline__ bool divides(float b) { return fabsf(b) > 1e-12f && fabsf(b) < 1e8f; }
+__device__ __forceinline__ bool divided(float a) { return fabsf(a) < 1e24f && (fabsf(a) > 1e-28f || a == 0.f); }
+__device__ __forceinline__ Divisor divisor(float b) { return Divisor{b, __fdiv_rn(1.f, b)}; }
+template <bool FAST>
+__device__ __forceinline__ float quotient(float a, const Divisor& d, bool& ok) {
+  if (!FAST) return __fdiv_rn(a, d.b);
+  ok = ok && divided(a);
+  float q = __fmul_rn(a, d.y);
+  q = __fmaf_rn(__fmaf_rn(-q, d.b, a), d.y, q);
+  return __fmaf_rn(__fmaf_rn(-q, d.b, a), d.y, q);
 }
 
-// W1: [N, ldw] block start (column i1), count <= 128 columns; a warp to a row, as many warps to a block as give every SM
-// its rows in one go.  Bound by the instructions of the serial chain, 128 columns of about 90 a warp: what a column's
-// owner need not know at once (the loss) is left to the end, and columns that are settled are not visited again (4096
-// rows: 117 -> 73 us, with 8 warps a block, a loss per column and all four column groups at each step before).
-constexpr int kMaxRowWarps = 16;
-__global__ void __launch_bounds__(32 * kMaxRowWarps)
-sparsegpt_block_kernel(const float* __restrict__ W, long long ldw, const float* __restrict__ hinv,
-                       long long ldh, const float* __restrict__ scale, const float* __restrict__ zero,
-                       float maxq, int N, int count, float* __restrict__ Q, float* __restrict__ Err,
-                       float* __restrict__ loss) {
-  extern __shared__ float s_h_raw[];                       // [128][128] floats
-  float (*s_h)[kCBlock] = reinterpret_cast<float (*)[kCBlock]>(s_h_raw);
-  for (int i = threadIdx.x; i < count * count; i += blockDim.x) {
-    const int r = i / count, c = i % count;
-    s_h[r][c] = c >= r ? hinv[(size_t)r * ldh + c] : 0.f;
+// One group of four columns of a row: ranked by w^2 / d^2, the two smallest pruned (ties: the lower column first, as a stable
+// selection does), each quantised (quant.py:9-18: q = clamp(round(w / scale) + zero, 0, maxq), scale * (q - zero)) and its
+// error fed forward to the group's later columns.  False: a division was outside the range of the quick form.
+struct Group {
+  float q[4], err[4], loss[4];
+};
+template <bool FAST>
+__device__ __forceinline__ bool settle_group(const float (&w0)[4], const float (&h)[4][4], const Divisor (&diag)[4],
+                                             const Divisor (&square)[4], const Divisor& scale, float zero, float maxq, Group& g) {
+  bool ok = true;
+  float w[4], rank[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    w[e] = w0[e];
+    rank[e] = quotient<FAST>(__fmul_rn(w[e], w[e]), square[e], ok);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    int smaller = 0;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) smaller += (rank[o] < rank[e] || (rank[o] == rank[e] && o < e)) ? 1 : 0;
+    const float code = rintf(quotient<FAST>(smaller < 2 ? 0.f : w[e], scale, ok)) + zero;
+    g.q[e] = __fmul_rn(scale.b, fminf(fmaxf(code, 0.f), maxq) - zero);
+    const float diff = w[e] - g.q[e];
+    g.err[e] = quotient<FAST>(diff, diag[e], ok);
+    g.loss[e] = __fmul_rn(diff, diff);
+    // W1[:, i:] -= err * Hinv1[i, i:] (the column itself is not read again)
+#pragma unroll
+    for (int o = e + 1; o < 4; ++o) w[o] = __fsub_rn(w[o], __fmul_rn(g.err[e], h[e][o]));
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) g.loss[e] = quotient<FAST>(g.loss[e], square[e], ok);
+  return ok;
+}
+
+// W1: [N, ldw] block start (column i1), count <= 128 columns.  Lane t of a row's T holds the groups G = T J + t: columns
+// 4 T J + 4 t + 0..3.  The chain -- rank, quantise, error, next column -- stays inside the lane that owns a group, the rows
+// of a warp side by side; its four errors then go to the row's other lanes, which take them off their later groups.
+// `w[0]` is the group of the current J (registers move down by one a J, so that the loop over the 32 groups is one body
+// of code).  Bound by the latency of that chain, which the divisions by the grid and by the diagonal make up: CUDA's
+// own, whose slow path a pruned entry's zero takes, cost 51 us a block of 4096 rows (T = 4), the quick form with a test for
+// each 43, with one test a group 33, and 31 with T = 8, two warps to a scheduler (T = 16: 37; a warp to a row, 73).
+constexpr int kRowLanes = 8, kBlockRows = 32;   // rows of a block: one block an SM for 4096 rows, three fit
+__global__ void __launch_bounds__(kRowLanes * kBlockRows)
+sparsegpt_block_kernel(const float* W, long long ldw, const float* __restrict__ hinv, long long ldh,
+                       const float* __restrict__ scale, const float* __restrict__ zero, float maxq, int N, int count,
+                       float* Q, long long ldq, float* __restrict__ Err, long long lde, float* __restrict__ loss) {
+  extern __shared__ __align__(16) float s_h[];             // [128][128]; what lies below a group of four is not read
+  if ((ldh & 3) == 0 && ((size_t)hinv & 15) == 0) {
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_h);
+    for (int i = threadIdx.x; i < kCBlock * kCBlock / 4; i += blockDim.x) {
+      const int r = i / (kCBlock / 4), c = i % (kCBlock / 4) * 4;
+      if (c + 3 >= r && c < count)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + i * 16), "l"(hinv + (size_t)r * ldh + c) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    for (int i = threadIdx.x; i < kCBlock * kCBlock; i += blockDim.x) {
+      const int r = i / kCBlock, c = i % kCBlock;
+      if (c >= r && c < count) s_h[i] = hinv[(size_t)r * ldh + c];
+    }
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= N) return;
-  const float sc = scale[row], zp = zero[row];
-  float w[4], q[4], e[4], diff[4], diag[4];
+  constexpr int T = kRowLanes, kGroups = kCBlock / (4 * T);
+  const int t = threadIdx.x & (T - 1);
+  const int place = blockIdx.x * kBlockRows + threadIdx.x / T;
+  const bool live = place < N;
+  const size_t row = live ? place : N - 1;                 // (whole warps take part in the exchange)
+  const Divisor sc = divisor(scale[row]);
+  const float zp = zero[row];
+  float w[kGroups][4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int c = lane + 32 * j;
-    w[j] = c < count ? W[(size_t)row * ldw + c] : 0.f;
-    diag[j] = c < count ? s_h[c][c] : 1.f;
-    q[j] = e[j] = diff[j] = 0.f;
-  }
+  for (int j = 0; j < kGroups; ++j)
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    bool pruned = false;
-    for (int l = 0; l < 32; ++l) {
-      const int i = 32 * j + l;
-      if (i >= count) break;
-      if ((i & 3) == 0) {
-        // the group's four columns live in lanes l .. l+3 (same j): rank by w^2 / d^2, prune
-        // the two smallest (ties: the lower column first, as a stable selection does)
-        const float mine = __fdiv_rn(__fmul_rn(w[j], w[j]), __fmul_rn(diag[j], diag[j]));
-        const int me = lane - l;
-        int smaller = 0;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float v = __shfl_sync(0xffffffffu, mine, (l + t) & 31);
-          smaller += (v < mine || (v == mine && t < me)) ? 1 : 0;
-        }
-        if (me >= 0 && me < 4) pruned = smaller < 2;
-      }
-      // column i: its owner lane quantises, everybody behind it receives the error
-      float err = 0.f;
-      if (lane == l) {
-        const float qi = quantize_sym(pruned ? 0.f : w[j], sc, zp, maxq);
-        q[j] = qi;
-        diff[j] = w[j] - qi;
-        err = __fdiv_rn(diff[j], diag[j]);
-        e[j] = err;
-      }
-      err = __shfl_sync(0xffffffffu, err, l);
-#pragma unroll
-      for (int jj = j; jj < 4; ++jj) {
-        const int c = lane + 32 * jj;
-        // W1[:, i:] -= err * Hinv1[i, i:]  (column i itself included, as in the reference)
-        if (c >= i && c < count) w[jj] = __fsub_rn(w[jj], __fmul_rn(err, s_h[i][c]));
-      }
+    for (int e = 0; e < 4; ++e) {
+      const int c = 4 * T * j + 4 * t + e;
+      w[j][e] = c < count ? W[row * ldw + c] : 0.f;
     }
-  }
   float row_loss = 0.f;
+  for (int J = 0; 4 * T * J < count; ++J) {
+    const int c0 = 4 * T * J + 4 * t;                      // this lane's group
+    float hb[4][4];
+    Divisor diag[4], square[4];
+    bool ranged = divides(sc.b);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int c = lane + 32 * j;
-    if (c < count) {
-      row_loss += __fdiv_rn(__fmul_rn(diff[j], diff[j]), __fmul_rn(diag[j], diag[j]));
-      Q[(size_t)row * count + c] = q[j];
-      Err[(size_t)row * count + c] = e[j];
+    for (int e = 0; e < 4; ++e) {
+      const float4 v = *reinterpret_cast<const float4*>(s_h + (c0 + e) * kCBlock + c0);
+      hb[e][0] = v.x; hb[e][1] = v.y; hb[e][2] = v.z; hb[e][3] = v.w;
+      diag[e] = divisor(hb[e][e]);
+      square[e] = divisor(__fmul_rn(hb[e][e], hb[e][e]));
+      ranged = ranged && divides(diag[e].b) && divides(square[e].b);
     }
+    for (int owner = 0; owner < T && 4 * T * J + 4 * owner < count; ++owner) {
+      Group g;
+      // (every lane goes through it; the owner's results count)
+      if (!(settle_group<true>(w[0], hb, diag, square, sc, zp, maxq, g) && ranged) && t == owner)
+        settle_group<false>(w[0], hb, diag, square, sc, zp, maxq, g);
+      float e4[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) e4[e] = __shfl_sync(0xffffffffu, g.err[e], owner, T);
+      if (t == owner && live) {
+        row_loss += (g.loss[0] + g.loss[1]) + (g.loss[2] + g.loss[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          Q[row * ldq + c0 + e] = g.q[e];
+          Err[row * lde + c0 + e] = g.err[e];
+        }
+      }
+      const float* h = s_h + (4 * T * J + 4 * owner) * kCBlock + c0;
+#pragma unroll
+      for (int j = 0; j < kGroups; ++j) {
+        if (4 * T * (J + j) >= count) break;
+        if (j == 0 && t <= owner) continue;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 v = *reinterpret_cast<const float4*>(h + e * kCBlock + 4 * T * j);
+          w[j][0] = __fsub_rn(w[j][0], __fmul_rn(e4[e], v.x));
+          w[j][1] = __fsub_rn(w[j][1], __fmul_rn(e4[e], v.y));
+          w[j][2] = __fsub_rn(w[j][2], __fmul_rn(e4[e], v.z));
+          w[j][3] = __fsub_rn(w[j][3], __fmul_rn(e4[e], v.w));
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j + 1 < kGroups; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[j][e] = w[j + 1][e];
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) row_loss += __shfl_xor_sync(0xffffffffu, row_loss, o);
-  if (lane == 0 && loss) loss[row] += row_loss * 0.5f;
+  for (int o = 1; o < T; o *= 2) row_loss += __shfl_xor_sync(0xffffffffu, row_loss, o);
+  if (t == 0 && live && loss) loss[row] += row_loss * 0.5f;
 }
 
 // one thread per packed word: grid covers [K*bits/32, N]
@@ -188,28 +253,25 @@ int dz_quant_find_params(const float* W, int N, int K, int bits, float* scale, f
   return DZ_OK;
 }
 
+int dz_sparsegpt_block_strided(const float* W_block, int64_t ldw, const float* hinv_block, int64_t ldh,
+                               const float* scale, const float* zero, int bits, int N, int count, float* Q,
+                               int64_t ldq, float* Err, int64_t lde, float* loss, void* stream) {
+  if (!W_block || !hinv_block || !scale || !zero || !Q || !Err) return DZ_ERR_INVALID_ARG;
+  if (N <= 0 || count <= 0 || count > kCBlock || (count & 3) || ldq < count || lde < count) return DZ_ERR_SHAPE;
+  if (bits != 2 && bits != 4 && bits != 8) return DZ_ERR_SHAPE;
+  constexpr int kSmem = kCBlock * kCBlock * sizeof(float);
+  DZ_CUDA_OK(cudaFuncSetAttribute(sparsegpt_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  sparsegpt_block_kernel<<<(N + kBlockRows - 1) / kBlockRows, kRowLanes * kBlockRows, kSmem, (cudaStream_t)stream>>>(
+      W_block, ldw, hinv_block, ldh, scale, zero, (float)((1 << bits) - 1), N, count, Q, ldq, Err, lde, loss);
+  DZ_CUDA_OK(cudaGetLastError());
+  return DZ_OK;
+}
+
 int dz_sparsegpt_block(const float* W_block, int64_t ldw, const float* hinv_block, int64_t ldh,
                        const float* scale, const float* zero, int bits, int N, int count, float* Q,
                        float* Err, float* loss, void* stream) {
-  if (!W_block || !hinv_block || !scale || !zero || !Q || !Err) return DZ_ERR_INVALID_ARG;
-  if (N <= 0 || count <= 0 || count > kCBlock || (count & 3)) return DZ_ERR_SHAPE;
-  if (bits != 2 && bits != 4 && bits != 8) return DZ_ERR_SHAPE;
-  constexpr int kSmem = kCBlock * kCBlock * sizeof(float);
-  static bool attr_set[64] = {};
-  int dev = 0;
-  DZ_CUDA_OK(cudaGetDevice(&dev));
-  if (!attr_set[dev & 63]) {
-    DZ_CUDA_OK(cudaFuncSetAttribute(sparsegpt_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    attr_set[dev & 63] = true;
-  }
-  int sms = 0;
-  DZ_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // two blocks to an SM where that takes all rows at once (three fit), and no fewer rows than make up for loading Hinv
-  const int per = N <= 4 * sms ? 4 : N <= 2 * sms * kMaxRowWarps ? (N + 2 * sms - 1) / (2 * sms) : kMaxRowWarps;
-  sparsegpt_block_kernel<<<(N + per - 1) / per, 32 * per, kSmem, (cudaStream_t)stream>>>(
-      W_block, ldw, hinv_block, ldh, scale, zero, (float)((1 << bits) - 1), N, count, Q, Err, loss);
-  DZ_CUDA_OK(cudaGetLastError());
-  return DZ_OK;
+  return dz_sparsegpt_block_strided(W_block, ldw, hinv_block, ldh, scale, zero, bits, N, count, Q, count, Err, count,
+                                    loss, stream);
 }
 
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,

@@ -293,6 +293,8 @@ int dz_paged_attention_decode(const void* qkv, int q_row_stride, void* out, cons
  *   ldh).  Writes Q [N, count] (pruned + quantised block) and Err [N, count] ((w - q) / Hinv_ii)
  *   and adds every row's loss to loss[n] (may be NULL).  The caller copies Q into W and applies
  *   W[:, i2:] -= Err @ Hinv[i1:i2, i2:] before the next block.  count % 4 == 0.
+ * dz_sparsegpt_block_strided: the same with rows of Q and Err ldq and lde elements apart; Q may be
+ *   W_block itself (ldq = ldw).
  * dz_pack_gptq: QuantLinear.pack (deltazip/nn_modules/qlinear.py:83-183, one group) of the
  *   quantised W [N, K]: qweight int32 [K*bits/32, N], qzeros int32 [1, N*bits/32], scales fp16
  *   [1, N] -- the tensors the reference stores and dz_convert_from_gptq reads.
@@ -301,6 +303,9 @@ int dz_quant_find_params(const float* W, int N, int K, int bits, float* scale, f
 int dz_sparsegpt_block(const float* W_block, int64_t ldw, const float* hinv_block, int64_t ldh,
                        const float* scale, const float* zero, int bits, int N, int count, float* Q,
                        float* Err, float* loss, void* stream);
+int dz_sparsegpt_block_strided(const float* W_block, int64_t ldw, const float* hinv_block, int64_t ldh,
+                               const float* scale, const float* zero, int bits, int N, int count, float* Q,
+                               int64_t ldq, float* Err, int64_t lde, float* loss, void* stream);
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,
                  int32_t* qweight, int32_t* qzeros, uint16_t* scales, void* stream);
 
