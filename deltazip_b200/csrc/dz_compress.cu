@@ -13,6 +13,7 @@
 //                            Outputs Q (quantised block) and Err ((w - q) / Hinv_ii per column),
 //                            from which the caller forms the update of the columns behind the
 //                            block, W[:, i2:] -= Err @ Hinv[i1:i2, i2:] (:146), a plain GEMM.
+//   triangular_inverse_kernel  the 128-wide diagonal blocks of an upper triangular matrix inverted, all in one launch.
 //   pack_gptq_kernel         QuantLinear.pack (deltazip/nn_modules/qlinear.py:83-183) for one
 //                            quantisation group: codes round((W + zero*scale) / fp16(scale))
 //                            packed along K into int32 words, zero points (minus one) packed
@@ -182,6 +183,51 @@ sparsegpt_block_kernel(const float* W, long long ldw, const float* __restrict__ 
   if (t == 0 && live && loss) loss[row] += row_loss * 0.5f;
 }
 
+// Diagonal blocks of 128 (the last may be smaller) of an upper triangular matrix inverted into `X`, whose other entries are
+// left alone.  Eight lanes own a column of the inverse, lane t the rows 8 m + t, and go up it: an entry once known is
+// handed to the other lanes, which take its share off their rows' sums -- sixteen independent sums a lane, so that a
+// step's latency is one exchange and one multiply-add, not a chain of them (four lanes with a sum each: 122 us for the 32
+// blocks of 4096 columns).  `acc[0]` belongs to the current m; sums move down by one each eight rows.
+constexpr int kInvLanes = 8, kInvRows = kCBlock / kInvLanes, kInvLd = kCBlock + 2;     // (eight rows: eight pairs of banks)
+__global__ void __launch_bounds__(kInvLanes * kCBlock)
+triangular_inverse_kernel(const double* __restrict__ R, long long ldr, int k, double* __restrict__ X, long long ldx) {
+  extern __shared__ double s[];                            // R, and below its diagonal the inverse, transposed
+  __shared__ double s_diag[kCBlock];                       // diagonal of the inverse
+  const int b0 = blockIdx.x * kCBlock, n = min(kCBlock, k - b0);
+  for (int i = threadIdx.x; i < kCBlock * kCBlock; i += blockDim.x) {
+    const int r = i / kCBlock, c = i % kCBlock;
+    if (c >= r) s[r * kInvLd + c] = c < n ? R[(size_t)(b0 + r) * ldr + b0 + c] : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < kCBlock) s_diag[threadIdx.x] = (int)threadIdx.x < n ? 1.0 / s[threadIdx.x * (kInvLd + 1)] : 0.0;
+  __syncthreads();
+  const int t = threadIdx.x & 7, col = threadIdx.x >> 3;
+  double acc[kInvRows];
+#pragma unroll
+  for (int m = 0; m < kInvRows; ++m) acc[m] = 0.0;
+  for (int M = kInvRows - 1; M >= 0; --M) {
+    for (int o = kInvLanes - 1; o >= 0; --o) {
+      const int l = 8 * M + o;
+      double x = l == col ? s_diag[l] : acc[0] * s_diag[l];          // (of lane o; zero below the diagonal: no sum yet)
+      x = __shfl_sync(0xffffffffu, x, o, kInvLanes);
+      if (t == o && l < col) s[col * kInvLd + l] = x;
+      if (t < o) acc[0] -= s[(8 * M + t) * kInvLd + l] * x;
+#pragma unroll
+      for (int m = 1; m < kInvRows; ++m) {
+        if (m > M) break;
+        acc[m] -= s[(8 * (M - m) + t) * kInvLd + l] * x;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m + 1 < kInvRows; ++m) acc[m] = acc[m + 1];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
+    const int r = i / n, c = i % n;
+    X[(size_t)(b0 + r) * ldx + b0 + c] = c > r ? s[c * kInvLd + r] : c == r ? s_diag[r] : 0.0;
+  }
+}
+
 // one thread per packed word: grid covers [K*bits/32, N]
 __global__ void pack_gptq_kernel(const float* __restrict__ Wq, const float* __restrict__ scale,
                                  const float* __restrict__ zero, int N, int K, int bits,
@@ -272,6 +318,16 @@ int dz_sparsegpt_block(const float* W_block, int64_t ldw, const float* hinv_bloc
                        float* Err, float* loss, void* stream) {
   return dz_sparsegpt_block_strided(W_block, ldw, hinv_block, ldh, scale, zero, bits, N, count, Q, count, Err, count,
                                     loss, stream);
+}
+
+int dz_triangular_inverse_blocks(const double* R, int64_t ldr, int k, double* X, int64_t ldx, void* stream) {
+  if (!R || !X) return DZ_ERR_INVALID_ARG;
+  if (k <= 0 || ldr < k || ldx < k) return DZ_ERR_SHAPE;
+  constexpr int kSmem = kCBlock * kInvLd * sizeof(double);
+  DZ_CUDA_OK(cudaFuncSetAttribute(triangular_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  triangular_inverse_kernel<<<(k + kCBlock - 1) / kCBlock, kInvLanes * kCBlock, kSmem, (cudaStream_t)stream>>>(R, ldr, k, X, ldx);
+  DZ_CUDA_OK(cudaGetLastError());
+  return DZ_OK;
 }
 
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,

@@ -295,6 +295,8 @@ int dz_paged_attention_decode(const void* qkv, int q_row_stride, void* out, cons
  *   W[:, i2:] -= Err @ Hinv[i1:i2, i2:] before the next block.  count % 4 == 0.
  * dz_sparsegpt_block_strided: the same with rows of Q and Err ldq and lde elements apart; Q may be
  *   W_block itself (ldq = ldw).
+ * dz_triangular_inverse_blocks: the 128 x 128 blocks on the diagonal of the upper triangular R [k, k]
+ *   (rows ldr elements apart), each inverted into the same place of X; a last block may be smaller.  Below the diagonal of a block X gets zeros, outside the blocks it is left alone.
  * dz_pack_gptq: QuantLinear.pack (deltazip/nn_modules/qlinear.py:83-183, one group) of the
  *   quantised W [N, K]: qweight int32 [K*bits/32, N], qzeros int32 [1, N*bits/32], scales fp16
  *   [1, N] -- the tensors the reference stores and dz_convert_from_gptq reads.
@@ -306,6 +308,7 @@ int dz_sparsegpt_block(const float* W_block, int64_t ldw, const float* hinv_bloc
 int dz_sparsegpt_block_strided(const float* W_block, int64_t ldw, const float* hinv_block, int64_t ldh,
                                const float* scale, const float* zero, int bits, int N, int count, float* Q,
                                int64_t ldq, float* Err, int64_t lde, float* loss, void* stream);
+int dz_triangular_inverse_blocks(const double* R, int64_t ldr, int k, double* X, int64_t ldx, void* stream);
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,
                  int32_t* qweight, int32_t* qzeros, uint16_t* scales, void* stream);
 

@@ -1,5 +1,6 @@
 """The compressor's kernels at their edges: one block of columns against the arithmetic step by step in numpy (bit for bit,
-in place and not, rows that do not fill a thread block, divisions outside the quick form's range)."""
+in place and not, rows that do not fill a thread block, divisions outside the quick form's range), and the inverses of
+diagonal blocks against 64 bits."""
 import numpy as np
 import pytest
 import torch
@@ -69,3 +70,23 @@ def test_one_block(n, count, lead, size):
         # `count` terms in 32 bits, each of them three roundings of its own
         true = (want_e.astype(np.float64) ** 2).sum(1) / 2
         assert (np.abs(loss - true) <= (count + 4) * 2.0 ** -23 * true + 1e-37).all()
+
+
+@pytest.mark.parametrize("k", [1, 7, 128, 129, 300, 512])
+def test_inverses_of_diagonal_blocks(k):
+    from deltazip_b200._lib import check, lib
+    g = torch.Generator().manual_seed(k)
+    R = torch.randn((k, k + 2), generator=g, dtype=torch.float64).cuda() * 0.1      # what lies below the diagonal is not read
+    R.diagonal().copy_(1 + torch.rand(k, generator=g, dtype=torch.float64))
+    X = torch.full((k, k), 9.0, dtype=torch.float64, device="cuda")
+    check(lib().dz_triangular_inverse_blocks(R.data_ptr(), k + 2, k, X.data_ptr(), k,
+                                             torch.cuda.current_stream().cuda_stream), "inverse")
+    for b in range(0, k, 128):
+        e = min(b + 128, k)
+        block, got = R[b:e, b:e].triu(), X[b:e, b:e]
+        assert not got.tril(-1).any()
+        # back substitution: a column's residual is below n * 2^-53 times |R| |X| (Higham, Accuracy and Stability, 8.5)
+        residual = (block @ got - torch.eye(e - b, dtype=torch.float64, device="cuda")).abs()
+        assert (residual <= (e - b + 2) * 2.0 ** -52 * (block.abs() @ got.abs())).all()
+        X[b:e, b:e] = 9
+    assert (X == 9).all()
