@@ -119,7 +119,8 @@ def hinv_factor(H: torch.Tensor, percdamp: float = 0.01) -> Tuple[torch.Tensor, 
     H[idx, idx] += damp
     R = torch.linalg.cholesky(H.mT.flip(0, 1).double()).flip(0, 1)
     dtype = R.dtype if _products_are_reduced(H) else H.dtype
-    inverse = _upper_inverse_cuda(R, dtype) if R.is_cuda else _upper_inverse(R.to(dtype))
+    # (a Hessian that carries gradients keeps the differentiable form)
+    inverse = _upper_inverse_cuda(R, dtype) if R.is_cuda and not R.requires_grad else _upper_inverse(R.to(dtype))
     return inverse.to(H.dtype).contiguous(), dead
 
 
@@ -174,7 +175,7 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
         if behind:
             check(L.dz_split_update(errors.data_ptr(), blocksize, n, count, hinv.data_ptr() + 4 * (i1 * k + i2), k, behind,
                                     left.data_ptr(), right.data_ptr(), _stream()), "dz_split_update")
-            later = W[:, i2:]
+            later = W.detach()[:, i2:]                           # (a product into `out` takes no gradients)
             torch.addmm(later, left[:6 * n * count].view(n, 6 * count), right[:6 * count * behind].view(6 * count, behind),
                         alpha=-1, out_dtype=torch.float32, out=later)
     return W, scale, zero, loss

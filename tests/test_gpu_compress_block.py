@@ -112,3 +112,16 @@ def test_operands_of_the_update(n, count, c):
     product = a.reshape(n, -1) @ b.reshape(-1, c)
     # what is left out: m l, l m and l l, and the splits' own rest
     assert ((product - e @ u).abs() <= 2.0 ** -23 * (e.abs() @ u.abs())).all()
+
+
+def test_inputs_that_carry_gradients():
+    from deltazip_b200 import compress
+    g = torch.Generator(device="cuda").manual_seed(0)
+    delta = torch.randn((32, 256), generator=g, device="cuda")
+    x = torch.randn((512, 256), generator=g, device="cuda")
+    H = x.t() @ x / 256
+    plain = compress.sparsegpt_2_4(delta, 4, H)
+    # the factor's other form differs by its roundings, and a code that lies between two values by one step
+    carried = compress.sparsegpt_2_4(delta.clone().requires_grad_(), 4, H.clone().requires_grad_())
+    assert (plain[0] != carried[0]).float().mean() <= 1e-3
+    torch.testing.assert_close(plain[3], carried[3].detach(), rtol=1e-2, atol=0)
