@@ -134,6 +134,15 @@ def find_params(W: torch.Tensor, bits: int) -> Tuple[torch.Tensor, torch.Tensor]
     return scale, zero
 
 
+def _without_slope(result: torch.Tensor, *inputs: torch.Tensor) -> torch.Tensor:
+    """`result` as a function of `inputs` that is constant around them, as a value on the quantisation grid is: gradients
+    of zero for those that carry one, which the kernels' writes through a pointer would not give by themselves."""
+    if not torch.is_grad_enabled() or not any(t.requires_grad for t in inputs):
+        return result
+    tied = result + sum(t.sum() for t in inputs if t.requires_grad)
+    return tied.copy_(result)
+
+
 def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = None,
                   percdamp: float = 0.01, blocksize: int = 128, hinv: Optional[torch.Tensor] = None):
     """2:4-pruned, `bits`-bit quantised delta with SparseGPT error feedback.
@@ -148,7 +157,7 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
     n, k = delta.shape
     if k % 4:
         raise ValueError("K must be a multiple of 4")
-    W = delta.clone().contiguous()
+    W = delta.detach().clone().contiguous()
     scale, zero = find_params(W, bits)
     if hinv is None:
         if H is None:
@@ -175,10 +184,10 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
         if behind:
             check(L.dz_split_update(errors.data_ptr(), blocksize, n, count, hinv.data_ptr() + 4 * (i1 * k + i2), k, behind,
                                     left.data_ptr(), right.data_ptr(), _stream()), "dz_split_update")
-            later = W.detach()[:, i2:]                           # (a product into `out` takes no gradients)
+            later = W[:, i2:]
             torch.addmm(later, left[:6 * n * count].view(n, 6 * count), right[:6 * count * behind].view(6 * count, behind),
                         alpha=-1, out_dtype=torch.float32, out=later)
-    return W, scale, zero, loss
+    return _without_slope(W, delta, hinv), scale, zero, loss
 
 
 def pack_gptq(Wq: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, bits: int):

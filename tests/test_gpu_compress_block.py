@@ -125,3 +125,23 @@ def test_inputs_that_carry_gradients():
     carried = compress.sparsegpt_2_4(delta.clone().requires_grad_(), 4, H.clone().requires_grad_())
     assert (plain[0] != carried[0]).float().mean() <= 1e-3
     torch.testing.assert_close(plain[3], carried[3].detach(), rtol=1e-2, atol=0)
+
+
+@pytest.mark.parametrize("of", ["delta", "H", "both"])
+def test_a_quantised_delta_has_no_slope(of):
+    """The result lies on a grid: its gradient is zero in the delta and in the Hessian, and its tangent is."""
+    from deltazip_b200 import compress
+    g = torch.Generator(device="cuda").manual_seed(1)
+    delta = torch.randn((32, 256), generator=g, device="cuda").requires_grad_(of != "H")
+    x = torch.randn((512, 256), generator=g, device="cuda")
+    H = (x.t() @ x / 256).requires_grad_(of != "delta")
+    Wq = compress.sparsegpt_2_4(delta, 4, H)[0]
+    (Wq * torch.randn(Wq.shape, generator=g, device="cuda")).sum().backward()
+    for t in (delta, H):
+        assert t.grad is None if not t.requires_grad else not t.grad.any()
+    with torch.no_grad():
+        assert not compress.sparsegpt_2_4(delta, 4, H)[0].requires_grad
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(delta.detach(), torch.ones_like(delta))
+        tangent = torch.autograd.forward_ad.unpack_dual(compress.sparsegpt_2_4(dual, 4, H.detach())[0]).tangent
+        assert tangent is None or not tangent.any()
