@@ -14,6 +14,8 @@ import math
 from typing import Optional, Tuple
 
 import torch
+import torch.autograd.forward_ad as forward_ad
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from ._lib import check, lib
 
@@ -95,6 +97,14 @@ def _upper_inverse_cuda(R: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return X
 
 
+def _only_values(t: torch.Tensor) -> bool:
+    """Whether nothing is asked of `t` but its values: no gradient, tangent or level of torch.func, no subclass, mode or
+    trace that follows the operations.  A kernel behind a pointer shows itself to none of those."""
+    return (type(t) is torch.Tensor and not t.requires_grad and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and forward_ad.unpack_dual(t).tangent is None and _get_current_dispatch_mode() is None
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 def _products_are_reduced(t: torch.Tensor) -> bool:
     """Whether the program lets 32-bit products of such matrices run at a lower precision (TF32, bf16)."""
     backend = torch.backends.cuda if t.is_cuda else torch.backends.mkldnn
@@ -119,8 +129,7 @@ def hinv_factor(H: torch.Tensor, percdamp: float = 0.01) -> Tuple[torch.Tensor, 
     H[idx, idx] += damp
     R = torch.linalg.cholesky(H.mT.flip(0, 1).double()).flip(0, 1)
     dtype = R.dtype if _products_are_reduced(H) else H.dtype
-    # (a Hessian that carries gradients keeps the differentiable form)
-    inverse = _upper_inverse_cuda(R, dtype) if R.is_cuda and not R.requires_grad else _upper_inverse(R.to(dtype))
+    inverse = _upper_inverse_cuda(R, dtype) if R.is_cuda and _only_values(R) else _upper_inverse(R.to(dtype))
     return inverse.to(H.dtype).contiguous(), dead
 
 

@@ -2,6 +2,7 @@
 and levels of the triangular inverse, a Hessian whose other triangle is not kept up, reduced-precision products."""
 import pytest
 import torch
+import torch.fx.experimental.proxy_tensor
 
 DEVICES = ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)]
 
@@ -63,3 +64,41 @@ def test_factor_where_products_may_be_reduced(precision, device):
     finally:
         torch.set_float32_matmul_precision(before)
     close(got, H, 0.05)
+
+
+def _derivatives(H, direction):
+    """What a trace and the forms of differentiation say of the factor: a trace, forward mode twice, backward mode twice
+    (which torch refuses above 512 columns, where the joined halves are written in place)."""
+    from deltazip_b200 import compress
+    factor = lambda h: compress.hinv_factor(h, 0.05)[0]
+    yield torch.fx.experimental.proxy_tensor.make_fx(factor)(H + torch.eye(len(H), dtype=H.dtype, device=H.device))(H)
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(H, direction)
+        tangent = torch.autograd.forward_ad.unpack_dual(factor(dual)).tangent
+        yield tangent.clone()
+    yield torch.func.jvp(factor, (H,), (direction,))[1]
+    if len(H) > 512:
+        return
+    yield torch.func.grad(lambda h: (factor(h) * direction).sum())(H)
+    leaf = H.clone().requires_grad_()
+    yield torch.autograd.grad((factor(leaf) * direction).sum(), leaf)[0]
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("k", [96, 256, 640])
+def test_derivatives_and_traces(k, device):
+    H = hessian(k, "cpu").double() + 0.1 * torch.eye(k, dtype=torch.float64)       # well conditioned, no dead column
+    direction = torch.randn((k, k), generator=torch.Generator().manual_seed(k), dtype=torch.float64)
+    direction = direction + direction.T
+    got = list(_derivatives(H.to(device), direction.to(device)))
+
+    def factor(h):                                 # (a damped H in terms of which torch differentiates the textbook's form)
+        h = h + 0.05 * h.diag().mean() * torch.eye(k, dtype=torch.float64)
+        return torch.linalg.cholesky(torch.linalg.inv(h), upper=True)
+    slope = torch.func.jvp(factor, (H,), (direction,))[1]
+    for tangent in got[1:3]:
+        torch.testing.assert_close(tangent.cpu(), slope, rtol=1e-7, atol=1e-9)      # 64 bits throughout
+    back = torch.func.grad(lambda h: (factor(h) * direction).sum())(H)
+    for gradient in got[3:]:                      # (only the lower triangle is read: its gradient along a symmetric direction)
+        torch.testing.assert_close((gradient.cpu() * direction).sum(), (back * direction).sum(), rtol=1e-7, atol=1e-9)
+    torch.testing.assert_close(got[0].cpu(), factor(H), rtol=1e-9, atol=1e-11)
