@@ -56,11 +56,11 @@ def _upper_inverse(R: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def _join_inverses(X: torch.Tensor, R: torch.Tensor, h: int, until: int) -> None:
+def _join_inverses(X: torch.Tensor, R: torch.Tensor, h: int) -> None:
     """X holds the inverses of R's diagonal blocks of h columns (the last may be smaller); pairs of them are joined
-    until the blocks have `until` columns."""
+    until one is left."""
     k = R.shape[0]
-    while h < min(k, until):
+    while h < k:
         first = 0
         if h < 1024:                                         # pairs of two whole halves: one batched product
             pairs = k // (2 * h)
@@ -84,16 +84,16 @@ def _join_inverses(X: torch.Tensor, R: torch.Tensor, h: int, until: int) -> None
         h *= 2
 
 
-def _upper_inverse_cuda(R: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-    """The same on the GPU for R in 64 bits: blocks of 128 by one launch, joined up to 512 columns in 64 bits and from
-    there on in `dtype` (4096 columns: 2.6 ms with library solves of 512, 1.1 ms so)."""
+def _upper_inverse_cuda(R: torch.Tensor) -> torch.Tensor:
+    """The same on the GPU for R in 64 bits: blocks of 128 by one launch, joined by products in 64 bits.  4096 columns
+    1.44 ms, 11008 21.6; as `_upper_inverse` in 32 bits 2.69 and 21.2, where the error against 64 bits is 3.7e-7 and 6.2e-7
+    (here that of rounding the result, 2.6e-8).  Joined in 32 bits above 512 columns 1.06 and 13.8 ms, but with a larger error
+    than that form's from about 2500 columns on (2944: 3.4e-7 and 3.3e-7, 11008: 6.7e-7)."""
     k = R.shape[0]
     R = R.contiguous()
     X = torch.zeros_like(R)
     check(lib().dz_triangular_inverse_blocks(R.data_ptr(), k, k, X.data_ptr(), k, _stream()), "dz_triangular_inverse_blocks")
-    _join_inverses(X, R, 128, 512)
-    X, R = X.to(dtype), R.to(dtype)
-    _join_inverses(X, R, 512, k)
+    _join_inverses(X, R, 128)
     return X
 
 
@@ -116,11 +116,12 @@ def hinv_factor(H: torch.Tensor, percdamp: float = 0.01) -> Tuple[torch.Tensor, 
 
     With J the reversal of rows and columns and J H J = L L^T, R = J L J is upper triangular and H = R R^T, so
     H^-1 = (R^-1)^T R^-1: the factor is R^-1.  One factorisation and a triangular inverse in place of two
-    factorisations and an inverse of H (4096 columns: 12.3 -> 4.6 ms).  Only H's lower triangle is read.  The
-    factorisation is in 64 bits, 0.4 ms more: its rounding in 32 turned more codes that lie between two values than
-    the older form did (loss of a 3072-column layer against 64 bits, ten of them: older 1.2e-4, 32 bits 3.0e-4, so
-    9e-5; 4096 columns 2.7e-4, 3.0e-4, 2.4e-4).  Where 32-bit products may be TF32, which also reaches the triangular
-    solve (factor off by 1e-3), the inverse is taken in 64 bits too (1.5 ms more)."""
+    factorisations and an inverse of H.  Only H's lower triangle is read.  The factorisation is in 64 bits (0.4 ms more at
+    4096 columns): its rounding in 32 turned more codes that lie between two values than the two factorisations did (loss of
+    a 3072-column layer against 64 bits, ten of them: those 1.2e-4, 32 bits 3.0e-4, so 9e-5; 4096 columns 2.7e-4, 3.0e-4,
+    2.4e-4).  So is the inverse on the GPU (`_upper_inverse_cuda`); on the CPU, and where more than values is asked for, it is
+    in H's type, but in 64 bits where 32-bit products may be TF32, which also reaches the triangular solve (factor off by
+    1e-3)."""
     H = H.clone()
     dead = torch.diag(H) == 0
     H[dead, dead] = 1
@@ -128,8 +129,10 @@ def hinv_factor(H: torch.Tensor, percdamp: float = 0.01) -> Tuple[torch.Tensor, 
     idx = torch.arange(H.shape[0], device=H.device)
     H[idx, idx] += damp
     R = torch.linalg.cholesky(H.mT.flip(0, 1).double()).flip(0, 1)
-    dtype = R.dtype if _products_are_reduced(H) else H.dtype
-    inverse = _upper_inverse_cuda(R, dtype) if R.is_cuda and _only_values(R) else _upper_inverse(R.to(dtype))
+    if R.is_cuda and _only_values(R):
+        inverse = _upper_inverse_cuda(R)
+    else:
+        inverse = _upper_inverse(R if _products_are_reduced(H) else R.to(H.dtype))
     return inverse.to(H.dtype).contiguous(), dead
 
 

@@ -102,3 +102,32 @@ def test_derivatives_and_traces(k, device):
     for gradient in got[3:]:                      # (only the lower triangle is read: its gradient along a symmetric direction)
         torch.testing.assert_close((gradient.cpu() * direction).sum(), (back * direction).sum(), rtol=1e-7, atol=1e-9)
     torch.testing.assert_close(got[0].cpu(), factor(H), rtol=1e-9, atol=1e-11)
+
+
+@pytest.mark.parametrize("k", [300, 1024, 1500, 2048, 2200])
+def test_joined_halves(k):
+    """Pairs of equal halves in a batch, large ones with a quarter of each factor left out, a last one of any size."""
+    from deltazip_b200 import compress
+    g = torch.Generator().manual_seed(k)
+    R = (torch.randn((k, k), generator=g, dtype=torch.float64) / k ** 0.5).triu(1) + 2 * torch.eye(k, dtype=torch.float64)
+    X = torch.zeros_like(R)
+    for b in range(0, k, 128):
+        e = min(b + 128, k)
+        X[b:e, b:e] = torch.linalg.solve_triangular(R[b:e, b:e], torch.eye(e - b, dtype=torch.float64), upper=True)
+    compress._join_inverses(X, R, 128)
+    assert not X.tril(-1).any()
+    # products of at most k terms, one level above the other, with an inverse whose norm is below one
+    torch.testing.assert_close(X @ R, torch.eye(k, dtype=torch.float64), rtol=0, atol=k * 2.0 ** -50)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [100, 640, 1536, 2200, 2944])
+def test_factor_to_the_last_bit_or_so(k):
+    """On the GPU all of it is in 64 bits, and what is off is the rounding of the result: half a unit of the last place."""
+    from deltazip_b200 import compress
+    H = hessian(k, "cuda")
+    H.diagonal().add_(0.05)                        # (damped beforehand: a mean of the diagonal is a sum in 32 bits)
+    got, _ = compress.hinv_factor(H, 0.0)
+    want = torch.linalg.cholesky(H.flip(0, 1).double()).flip(0, 1)
+    want = torch.linalg.solve_triangular(want, torch.eye(k, dtype=torch.float64, device="cuda"), upper=True)
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24
