@@ -131,3 +131,12 @@ def test_factor_to_the_last_bit_or_so(k):
     want = torch.linalg.cholesky(H.flip(0, 1).double()).flip(0, 1)
     want = torch.linalg.solve_triangular(want, torch.eye(k, dtype=torch.float64, device="cuda"), upper=True)
     assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("k", [64, 640])
+def test_a_hessian_of_16_bits_is_refused(k, dtype, device):
+    from deltazip_b200 import compress
+    with pytest.raises(RuntimeError, match="not implemented"):
+        compress.hinv_factor((torch.eye(k) * 2).to(device, dtype))
