@@ -129,7 +129,7 @@ def hinv_factor(H: torch.Tensor, percdamp: float = 0.01) -> Tuple[torch.Tensor, 
     idx = torch.arange(H.shape[0], device=H.device)
     H[idx, idx] += damp
     R = torch.linalg.cholesky(H.mT.flip(0, 1).double()).flip(0, 1)
-    if R.is_cuda and _only_values(R) and H.dtype in (torch.float32, torch.float64):
+    if R.is_cuda and R.numel() and _only_values(R) and H.dtype in (torch.float32, torch.float64):
         inverse = _upper_inverse_cuda(R)
     else:
         inverse = _upper_inverse(R if _products_are_reduced(H) else R.to(H.dtype))

@@ -140,3 +140,10 @@ def test_a_hessian_of_16_bits_is_refused(k, dtype, device):
     from deltazip_b200 import compress
     with pytest.raises(RuntimeError, match="not implemented"):
         compress.hinv_factor((torch.eye(k) * 2).to(device, dtype))
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_no_columns(device):
+    from deltazip_b200 import compress
+    factor, dead = compress.hinv_factor(torch.empty((0, 0), device=device))
+    assert factor.shape == (0, 0) and dead.shape == (0,)
