@@ -92,7 +92,8 @@ def _upper_inverse_cuda(R: torch.Tensor) -> torch.Tensor:
     k = R.shape[0]
     R = R.contiguous()
     X = torch.zeros_like(R)
-    check(lib().dz_triangular_inverse_blocks(R.data_ptr(), k, k, X.data_ptr(), k, _stream()), "dz_triangular_inverse_blocks")
+    with torch.cuda.device(R.device):                        # (any, as for the library's calls)
+        check(lib().dz_triangular_inverse_blocks(R.data_ptr(), k, k, X.data_ptr(), k, _stream()), "dz_triangular_inverse_blocks")
     _join_inverses(X, R, 128)
     return X
 

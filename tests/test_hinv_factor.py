@@ -147,3 +147,12 @@ def test_no_columns(device):
     from deltazip_b200 import compress
     factor, dead = compress.hinv_factor(torch.empty((0, 0), device=device))
     assert factor.shape == (0, 0) and dead.shape == (0,)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="two GPUs")
+def test_factor_on_a_gpu_that_is_not_the_current_one():
+    from deltazip_b200 import compress
+    H = hessian(300, "cuda:1")
+    got, _ = compress.hinv_factor(H, 0.05)
+    close(got, H, 0.05)
