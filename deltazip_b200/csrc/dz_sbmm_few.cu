@@ -163,6 +163,8 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) sbmm_few_kernel(const 
     }
     if (bad) {                                                 // (the same in every thread)
       if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(p.status, 0, (int)DZ_ERR_INVALID_ARG);
+      // a grid that ended before its predecessor would let its successor start beside that
+      if (p.stable) asm volatile("griddepcontrol.wait;" ::: "memory");
       return;
     }
     __syncthreads();

@@ -496,8 +496,10 @@ sbmm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   if (bad) {
     // rejected batch: nothing runs, but the tiles requested in the prologue must land before
-    // this CTA's shared memory is released
+    // this CTA's shared memory is released, and the predecessor must have ended before this grid does: its end is all
+    // that the successor waits for
     if (threadIdx.x == 0) {
+      if (p.stable) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < npre_x; ++i) mbar_wait(smem_u32(&bar_x_full[i]), 0, abort_flag, nullptr);
       if (!p.delta_only)
         for (int i = 0; i < npre_w; ++i) mbar_wait(smem_u32(&bar_w_full[i]), 0, abort_flag, nullptr);

@@ -85,3 +85,31 @@ def test_wrong_promise_is_reported_and_y_left():
     ops.sbmm(dev(x), layer.qweight, layer.scales, layer.meta, seg, layer.w, out=y)
     assert ops.read_status() == _lib.DZ_ERR_INVALID_ARG
     assert (y == 5).all()
+
+
+@pytest.mark.parametrize("m,slots", [(6, 3), (32, 3)])
+def test_rejected_among_early_starting_calls(m, slots):
+    """Calls that start under their predecessor's tail, each reading what the one before wrote, with a rejected table in
+    between: its grid ends no sooner than the call before it, and the chain goes on.  (32 tokens: the form for larger batches.)"""
+    from deltazip_b200 import _lib, ops
+    layer = DeviceLayer(256, 256, slots, 4, seed=m)
+    x_np, idx = O.make_tokens(m, 256, slots, seed=m, sort=False, base_frac=0.2)
+    idx[:2] = [2, 0]
+    index = torch.from_numpy(idx).cuda()
+    seg = ops.Segments(m, slots, "cuda").build(index)
+    wrong = ops.Segments(m, slots, "cuda").build(index, sorted_hint=True)
+
+    def chain(reject):
+        x, ys = dev(x_np), [torch.full((m, 256), 5.0, dtype=torch.float16, device="cuda") for _ in range(12)]
+        torch.cuda.synchronize()                     # table, slots and weight are written before the chain begins
+        for y, kept in zip(ys[::2], ys[1::2]):
+            ops.sbmm(x, layer.qweight, layer.scales, layer.meta, seg, layer.w, out=y, stable=True)
+            if reject:
+                ops.sbmm(y, layer.qweight, layer.scales, layer.meta, wrong, layer.w, out=kept, stable=True)
+            x = y
+        return ys
+    ops.read_status()
+    want, got = chain(False), chain(True)
+    assert want[0].any() and torch.isfinite(want[10]).all()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    assert ops.read_status() == _lib.DZ_ERR_INVALID_ARG and ops.read_status() == 0
