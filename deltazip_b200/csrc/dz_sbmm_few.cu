@@ -119,10 +119,11 @@ struct Fields {
   }
 };
 
-// Bytes of a stage and stages of a warp's ring for slices of RT x 16 features, so that sixteen warps with their sums fit an SM.
+// Bytes of a stage and stages of a warp's ring for slices of RT x 16 features: sixteen warps of an SM have 192 KB in all
+// cases.  A warp's sums take the place of the stage that it has read last.
 __host__ __device__ constexpr int few_stage(int rt) { return rt * 16 * 128; }
 __host__ __device__ constexpr int few_depth(int rt) { return rt == 1 ? 6 : 3; }
-constexpr int few_smem(int rt, int nb, int warps) { return warps * (few_depth(rt) * few_stage(rt) + 8 * nb * rt * 16 * 4); }
+constexpr int few_smem(int rt, int warps) { return warps * few_depth(rt) * few_stage(rt); }
 
 // NB: blocks of eight tokens; RT: tiles of 16 features of a slice
 template <int BITS, int DT, int NB, int RT, int WARPS>
@@ -131,11 +132,13 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) sbmm_few_kernel(const 
   constexpr int kCodeBytes = kSlice * 4 * BITS, kMetaSlice = kSlice * 8;
   constexpr int kWin = kCodeBytes + kMetaSlice;                // one delta's part of a stage
   constexpr int kPieces = kWin / 16, kRounds = (kPieces + 31) / 32;
-  static_assert(kPerStage * kWin <= kStage, "stage");
+  static_assert(kPerStage * kWin <= kStage && 8 * NB * kSlice * 4 <= kStage, "stage");
   extern __shared__ __align__(128) uint8_t s_few[];
   __shared__ int s_slot[kFewMax], s_win[kFewMax];              // slot of each token, of each present delta
   __shared__ const uint8_t* s_from[kFewMax][2];                // codes and metadata of each present delta
-  float* const s_sum = reinterpret_cast<float*>(s_few + kFewWarps * D * kStage);
+  __shared__ int s_sum[WARPS];                                 // byte offset of each warp's sums
+  static_assert(16 / WARPS * (few_smem(RT, WARPS) + 2 * sizeof(int) * kFewMax + sizeof(s_from) + sizeof(s_sum) + 1024) <= 228 * 1024,
+                "sixteen warps an SM (1 KB of a CTA's shared memory is the system's)");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 
   if (!p.stable) {
@@ -353,8 +356,11 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) sbmm_few_kernel(const 
         }
       }
     }
-    // ---- the warps' sums, with their deltas' scales: [warp][column][row] ----
-    float* const mine = s_sum + warp * 8 * NB * kSlice;
+    // ---- the warps' sums, with their deltas' scales: [column][row], in the stage that the warp requests next ----
+    __syncwarp();                                              // (every lane has read it; nothing is under way to it)
+    const int mine_at = (warp * D + c_at) * kStage;
+    float* const mine = reinterpret_cast<float*>(s_few + mine_at);
+    if (lane == 0) s_sum[warp] = mine_at;
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) sbmm_few_kernel(const 
     for (int i = threadIdx.x; i < p.M * kSlice; i += 32 * kFewWarps) {
       float v = 0.f;
 #pragma unroll
-      for (int w = 0; w < kFewWarps; ++w) v += s_sum[w * 8 * NB * kSlice + i];
+      for (int w = 0; w < kFewWarps; ++w) v += reinterpret_cast<const float*>(s_few + s_sum[w])[i];
       store_out<DT>(p.y, (size_t)(i / kSlice) * p.ldy + slice * kSlice + i % kSlice, v, p.accumulate);
     }
     __syncthreads();
@@ -429,18 +435,25 @@ int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status,
   // two CTAs an SM have one each; narrower ones keep more SMs busy (one token, one delta: 4096 x 4096 10.3 us with 16, 11.1
   // with 32; 12288 x 4096 31.2 and 24.4).  Two CTAs of eight warps an SM; four of four where the slices are more than those.
   const int rt = a.N / 16 > 2 * sms ? 2 : 1, slices = a.N / (16 * rt), warps = slices > 2 * sms ? 4 : 8;
-  const int kidx = (a.bits == 4) + 2 * dt + 4 * nb + (warps == 4 ? 8 : 0) + 16 * (rt - 1), smem = few_smem(rt, nb + 1, warps);
+  // Three of those, held down to that by their shared memory, where rounds of three end sooner than rounds of four: with
+  // four some SMs get four CTAs and others two.  Base products of 9 rows, three always (four did not fit) and so: 11264 x
+  // 2048 10.7 us both, 22016 x 4096 35.4 and 34.4 (four: 38.6), 15360 x 5120 39.6 and 28.2, 32000 x 4096 50.9 and 44.3.
+  auto rounds = [&](int per_sm) { return (slices + per_sm * sms - 1) / (per_sm * sms); };
+  const int per_sm = warps == 8 ? 2 : 3 * rounds(3) < 4 * rounds(4) ? 3 : 4;
+  const int kidx = (a.bits == 4) + 2 * dt + 4 * nb + (warps == 4 ? 8 : 0) + 16 * (rt - 1);
+  constexpr int kAFourth = 228 * 1024 / 4;
+  const int smem = per_sm == 3 ? kAFourth : few_smem(rt, warps);
   Kern kern = kerns[kidx];
   static bool attr_set[64][32] = {};
   int dev = 0;
   DZ_CUDA_OK(cudaGetDevice(&dev));
   bool& set = attr_set[dev & 63][kidx];
   if (!set) {
-    DZ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    DZ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max(smem, kAFourth)));
     set = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(min(slices, 16 / warps * sms));
+  cfg.gridDim = dim3(min(slices, per_sm * sms));
   cfg.blockDim = dim3(32 * warps);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

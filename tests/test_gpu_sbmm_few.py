@@ -46,6 +46,21 @@ def test_bf16_and_base_alone(n, m):
     assert ((want - y.double()).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -10 * want.abs().max()).all()
 
 
+@pytest.mark.parametrize("bits", [4, 2])
+@pytest.mark.parametrize("k,m", [(64, 2), (192, 7), (320, 16), (384, 9)])
+def test_second_slices(k, m, bits):
+    """More slices of 32 features than four CTAs on each of 148 SMs: a CTA goes on to a second one, its rings as they are."""
+    n = 19328                                        # 604 slices
+    layer = DeviceLayer(n, k, 2, bits, seed=m)
+    x, idx = O.make_tokens(m, k, 2, seed=k, sort=False, base_frac=0.2)
+    y, _ = run_sbmm(layer, x, idx)
+    check(layer, x, idx, y)
+    from deltazip_b200 import ops
+    alone = ops.base_gemm(dev(x), layer.w)
+    base, _ = run_sbmm(layer, x, np.full(m, -1))
+    np.testing.assert_array_equal(alone.cpu().numpy().view(np.uint16), base.view(np.uint16))
+
+
 def test_columns_do_not_see_each_other():
     layer = DeviceLayer(256, 256, 4, 4, seed=1)
     x, _ = O.make_tokens(12, 256, 4, seed=1)
