@@ -34,7 +34,7 @@ constexpr int kPerStage = 5;                   // deltas of a stage
 constexpr int kFewMax = 16;                    // tokens, and so present deltas
 
 struct FewParams {
-  int M, N, K, num_slots, base_only, delta_only, tokens_sorted, accumulate, stable;
+  int M, N, K, num_slots, delta_only, tokens_sorted, accumulate, stable;
   long long ldy, qstride, mstride, sstride;
   const uint8_t *x, *w, *qweight, *meta, *scales, *seg;
   void* y;
@@ -412,7 +412,6 @@ bool sbmm_few_supported(const dz_sbmm_args& a, bool base_only) {
 int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status, cudaStream_t st) {
   FewParams p;
   p.M = a.M; p.N = a.N; p.K = a.K; p.num_slots = a.num_slots;
-  p.base_only = base_only;
   p.delta_only = !base_only && !a.w_base;
   p.tokens_sorted = base_only || a.tokens_sorted;
   p.accumulate = (a.flags & DZ_SBMM_ACCUMULATE) ? 1 : 0;
@@ -428,8 +427,7 @@ int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status,
   using Kern = void (*)(const FewParams);
 #define DZ_FEW(NB, RT, W) \
   sbmm_few_kernel<2, 0, NB, RT, W>, sbmm_few_kernel<4, 0, NB, RT, W>, sbmm_few_kernel<2, 1, NB, RT, W>, sbmm_few_kernel<4, 1, NB, RT, W>
-  static const Kern kerns[32] = {DZ_FEW(1, 1, 8), DZ_FEW(2, 1, 8), DZ_FEW(1, 1, 4), DZ_FEW(2, 1, 4),
-                                 DZ_FEW(1, 2, 8), DZ_FEW(2, 2, 8), DZ_FEW(1, 2, 4), DZ_FEW(2, 2, 4)};
+  static const Kern kerns[24] = {DZ_FEW(1, 1, 8), DZ_FEW(2, 1, 8), DZ_FEW(1, 2, 8), DZ_FEW(2, 2, 8), DZ_FEW(1, 2, 4), DZ_FEW(2, 2, 4)};
 #undef DZ_FEW
   // Slices of 32 features, with half the work per delta that does not grow with the features (metadata, masking x), where
   // two CTAs an SM have one each; narrower ones keep more SMs busy (one token, one delta: 4096 x 4096 10.3 us with 16, 11.1
@@ -440,11 +438,11 @@ int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status,
   // 2048 10.7 us both, 22016 x 4096 35.4 and 34.4 (four: 38.6), 15360 x 5120 39.6 and 28.2, 32000 x 4096 50.9 and 44.3.
   auto rounds = [&](int per_sm) { return (slices + per_sm * sms - 1) / (per_sm * sms); };
   const int per_sm = warps == 8 ? 2 : 3 * rounds(3) < 4 * rounds(4) ? 3 : 4;
-  const int kidx = (a.bits == 4) + 2 * dt + 4 * nb + (warps == 4 ? 8 : 0) + 16 * (rt - 1);
+  const int kidx = (a.bits == 4) + 2 * dt + 4 * nb + 8 * (rt - 1) + (warps == 4 ? 8 : 0);   // (four warps: slices of 32)
   constexpr int kAFourth = 228 * 1024 / 4;
   const int smem = per_sm == 3 ? kAFourth : few_smem(rt, warps);
   Kern kern = kerns[kidx];
-  static bool attr_set[64][32] = {};
+  static bool attr_set[64][24] = {};
   int dev = 0;
   DZ_CUDA_OK(cudaGetDevice(&dev));
   bool& set = attr_set[dev & 63][kidx];
