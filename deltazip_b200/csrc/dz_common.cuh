@@ -163,7 +163,7 @@ size_t sbmm_workspace_bytes(int M, int N, int K, int tokens_sorted);
 int check_sbmm_args(const dz_sbmm_args* a, bool base_only, bool check_workspace);
 int launch_sbmm(const dz_sbmm_args& a, bool base_only, cudaStream_t st);
 // The form for at most 16 tokens (no workspace but the status word).
-bool sbmm_few_supported(const dz_sbmm_args& a, bool base_only);
+bool sbmm_few_supported(const dz_sbmm_args& a, bool base_only, int sms);
 int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status, cudaStream_t st);
 // Delta products of a prompt batch added to y; xsrc: the tokens in sorted order.
 constexpr int kPrefillMaxSlots = 1024;     // three ints of shared memory per slot

@@ -1090,7 +1090,7 @@ int launch_sbmm(const dz_sbmm_args& a, bool base_only, cudaStream_t st) {
   if (a.N / kTileN > (int)(kWsCountersBytes / 8)) return DZ_ERR_TOO_LARGE;
 
   uint8_t* ws = reinterpret_cast<uint8_t*>(a.workspace);
-  if (sbmm_few_supported(a, base_only))
+  if (sbmm_few_supported(a, base_only, di.sms))
     return launch_sbmm_few(a, base_only, di.sms, reinterpret_cast<int*>(ws + kWsStatus), st);
   const bool sorted = base_only || a.tokens_sorted != 0;
   const void* xsrc = a.x;
