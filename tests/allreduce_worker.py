@@ -135,7 +135,7 @@ def main():
 
     # --- fused form: the SBMM epilogue pushes its tiles to every rank, the reduction sums local
     #     slots; same rounding as the separate all-reduce, so the outputs are bit-identical ---
-    for m2, sort in ((48, True), (300, True), (77, False)):
+    for m2, sort in ((48, True), (300, True), (77, False), (12, False)):
         x2 = torch.randn(m2, k, generator=gen, device=dev).half()
         idx2 = torch.randint(-1, slots, (m2,), generator=gen, device=dev)
         if sort:
@@ -148,7 +148,10 @@ def main():
         layers.RowParallelLinearWithDelta.FUSED_ALL_REDUCE = True
         for rep in range(6):                      # repeated: slots and flags alternate correctly
             y_fused = layer(xs)[0]
-            assert torch.equal(y_fused, y_sep), (m2, sort, rep, (y_fused.float() - y_sep.float()).abs().max())
+            if m2 > 16:
+                assert torch.equal(y_fused, y_sep), (m2, sort, rep, (y_fused.float() - y_sep.float()).abs().max())
+            else:                                 # (a product that is not pushed has a form, and an order of sums, of its own)
+                assert ((y_fused.float() - y_sep.float()).norm() / y_sep.float().norm()).item() < 1e-3
             if rep % 2:                           # interleave with reductions of the other kind
                 assert torch.equal(layer_sep_call(layer, xs), y_sep)
         ref2 = ops.apply_delta(x2, full[0], full[2], full[1], idx2, w).float()
