@@ -160,6 +160,8 @@ _SIGNATURES = {
                                            c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p]),
     "dz_triangular_inverse_blocks": (c_int, [c_void_p, c_int64, c_int, c_void_p, c_int64, c_void_p]),
     "dz_split_update": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p]),
+    "dz_split_update_rows": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_void_p,
+                                     c_void_p, c_void_p]),
     "dz_pack_gptq": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
                              c_void_p, c_void_p]),
     "dz_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]),

@@ -237,33 +237,69 @@ triangular_inverse_kernel(const double* __restrict__ R, long long ldr, int k, do
 // [h m l h m h] of U.  For a block of 128 columns the product's error against 64 bits is below that of a 32-bit GEMM (4096
 // rows: 1.2e-7 and 2.0e-7 of its norm; over 512 columns it would not be: 4.7e-7 and 4.1e-7, sums being cut, not rounded).
 // 4096 rows and 2048 columns behind the block: 55 us as a 32-bit GEMM, 16 so and 4 for this kernel, bound by its bytes.
+//   Range.  bf16 has the exponents of a float, so below 2^-109 a third part loses bits, and infinities leave NaN in the
+// others.  A row of E whose largest entry is outside [2^-64, 2^32], or not a number, is given zeros as operands and taken off
+// its row of W here, in 32 bits.  Of the other rows the parts' absolute error, 2^-134, is 2^-70 of the largest entry, and U's,
+// times E, below 2^-102.  A finite entry that rounds to infinity keeps the largest bf16 number as its first part.
 __device__ __forceinline__ void split3(float x, __nv_bfloat16* v) {
   v[0] = __float2bfloat16_rn(x);
+  if (__hisinf(v[0]) && fabsf(x) <= 3.4028235e38f) v[0] = __ushort_as_bfloat16(x > 0.f ? 0x7f7f : 0xff7f);
   const float r = x - __bfloat162float(v[0]);
   v[1] = __float2bfloat16_rn(r);
   v[2] = __float2bfloat16_rn(r - __bfloat162float(v[1]));
 }
-__global__ void split_update_kernel(const float* __restrict__ E, long long lde, int n, int count, const float* __restrict__ U,
-                                    long long ldu, int c, __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B) {
-  const long long left = (long long)n * (count / 4), all = left + (long long)count * (c / 4);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < all; i += (long long)gridDim.x * blockDim.x) {
-    const bool a = i < left;
-    const long long j = a ? i : i - left;
-    const int quads = (a ? count : c) / 4;
-    const long long row = j / quads, col = j % quads * 4;
-    const float* src = a ? E + row * lde + col : U + row * ldu + col;
-    __nv_bfloat16 v[4][3];
+// four entries into their six places, `part_of` giving the part of each
+template <typename F>
+__device__ __forceinline__ void store_parts(const float (&x)[4], __nv_bfloat16* dst, long long step, F part_of) {
+  __nv_bfloat16 v[4][3];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) split3(src[q], v[q]);
+  for (int q = 0; q < 4; ++q) split3(x[q], v[q]);
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
-      const int part = a ? (p == 0 ? 2 : p == 1 || p == 3 ? 1 : 0) : (p == 2 ? 2 : p == 1 || p == 4 ? 1 : 0);
-      __nv_bfloat16* dst = a ? A + (row * 6 + p) * count + col : B + ((long long)p * count + row) * c + col;
-      __nv_bfloat162 lo, hi;
-      lo.x = v[0][part]; lo.y = v[1][part];
-      hi.x = v[2][part]; hi.y = v[3][part];
-      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  for (int p = 0; p < 6; ++p) {
+    const int part = part_of(p);
+    __nv_bfloat162 lo, hi;
+    lo.x = v[0][part]; lo.y = v[1][part];
+    hi.x = v[2][part]; hi.y = v[3][part];
+    *reinterpret_cast<uint2*>(dst + p * step) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+// A warp takes a row of E, then quads of U.  W (may be null: every row is split): [n, c], the columns behind the block.
+__global__ void __launch_bounds__(256)
+split_update_kernel(const float* __restrict__ E, long long lde, int n, int count, const float* __restrict__ U, long long ldu, int c,
+                    float* W, long long ldw, __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < n; row += warps) {
+    const float* src = E + row * lde;
+    bool in = true, large = false, any = false;
+    if (W) {
+      for (int i = lane; i < count; i += 32) {
+        const float x = fabsf(src[i]);
+        in = in && x <= 0x1p32f;                             // (false for a NaN)
+        large = large || x >= 0x1p-64f;
+        any = any || x != 0.f;
+      }
+      in = __all_sync(0xffffffffu, in) && (__any_sync(0xffffffffu, large) || !__any_sync(0xffffffffu, any));
     }
+    for (int col = 4 * lane; col < count; col += 128) {
+      float x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = in ? src[col + q] : 0.f;
+      store_parts(x, A + (long long)row * 6 * count + col, count, [](int p) { return p == 0 ? 2 : p == 1 || p == 3 ? 1 : 0; });
+    }
+    if (!in)
+      for (int j = lane; j < c; j += 32) {
+        float sum = 0.f;
+        for (int i = 0; i < count; ++i) sum = fmaf(src[i], U[i * ldu + j], sum);
+        W[row * ldw + j] -= sum;
+      }
+  }
+  const long long quads = c / 4, all = count * quads;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < all; i += (long long)gridDim.x * blockDim.x) {
+    const long long row = i / quads, col = i % quads * 4;
+    float x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = U[row * ldu + col + q];
+    store_parts(x, B + row * c + col, (long long)count * c, [](int p) { return p == 2 ? 2 : p == 1 || p == 4 ? 1 : 0; });
   }
 }
 
@@ -369,16 +405,22 @@ int dz_triangular_inverse_blocks(const double* R, int64_t ldr, int k, double* X,
   return DZ_OK;
 }
 
-int dz_split_update(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, void* A, void* B,
-                    void* stream) {
+int dz_split_update_rows(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, float* W, int64_t ldw,
+                         void* A, void* B, void* stream) {
   if (!E || !U || !A || !B) return DZ_ERR_INVALID_ARG;
-  if (n <= 0 || count <= 0 || c <= 0 || (count & 3) || (c & 3) || lde < count || ldu < c) return DZ_ERR_SHAPE;
+  if (n <= 0 || count <= 0 || c <= 0 || (count & 3) || (c & 3) || lde < count || ldu < c || (W && ldw < c)) return DZ_ERR_SHAPE;
   if (((uintptr_t)A | (uintptr_t)B) & 7) return DZ_ERR_ALIGNMENT;
-  const long long quads = (long long)n * (count / 4) + (long long)count * (c / 4);
-  const int blocks = (int)(quads / 256 + 1 < 2048 ? quads / 256 + 1 : 2048);
-  split_update_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(E, lde, n, count, U, ldu, c, (__nv_bfloat16*)A, (__nv_bfloat16*)B);
+  const long long quads = max((long long)n * 32, (long long)count * (c / 4));
+  const int blocks = (int)min(quads / 256 + 1, 2048ll);
+  split_update_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(E, lde, n, count, U, ldu, c, W, ldw, (__nv_bfloat16*)A,
+                                                                (__nv_bfloat16*)B);
   DZ_CUDA_OK(cudaGetLastError());
   return DZ_OK;
+}
+
+int dz_split_update(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, void* A, void* B,
+                    void* stream) {
+  return dz_split_update_rows(E, lde, n, count, U, ldu, c, nullptr, 0, A, B, stream);
 }
 
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,

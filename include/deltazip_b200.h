@@ -300,6 +300,9 @@ int dz_paged_attention_decode(const void* qkv, int q_row_stride, void* out, cons
  * dz_split_update: operands for W -= E U as one bf16 GEMM with 32-bit sums: A [n, 6 count] holds rows
  *   [l m h m h h] of E [n, count], B [6 count, c] the rows [h m l h m h] of U [count, c], a float being
  *   h + m + l with three bf16 numbers (A B is then E U but for terms of 2^-24).  count and c in fours.
+ * dz_split_update_rows: the same; rows of E whose entries are outside the range where three bf16 numbers hold a
+ *   float (below 2^-64 in all, one above 2^32 or not finite) are zero in A, and W [n, c] (rows ldw elements
+ *   apart) has their share taken off in 32 bits.  W NULL: no row is treated so.
  * dz_pack_gptq: QuantLinear.pack (deltazip/nn_modules/qlinear.py:83-183, one group) of the
  *   quantised W [N, K]: qweight int32 [K*bits/32, N], qzeros int32 [1, N*bits/32], scales fp16
  *   [1, N] -- the tensors the reference stores and dz_convert_from_gptq reads.
@@ -314,6 +317,8 @@ int dz_sparsegpt_block_strided(const float* W_block, int64_t ldw, const float* h
 int dz_triangular_inverse_blocks(const double* R, int64_t ldr, int k, double* X, int64_t ldx, void* stream);
 int dz_split_update(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, void* A, void* B,
                     void* stream);
+int dz_split_update_rows(const float* E, int64_t lde, int n, int count, const float* U, int64_t ldu, int c, float* W, int64_t ldw,
+                         void* A, void* B, void* stream);
 int dz_pack_gptq(const float* Wq, const float* scale, const float* zero, int N, int K, int bits,
                  int32_t* qweight, int32_t* qzeros, uint16_t* scales, void* stream);
 

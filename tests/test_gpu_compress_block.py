@@ -145,3 +145,55 @@ def test_a_quantised_delta_has_no_slope(of):
         dual = torch.autograd.forward_ad.make_dual(delta.detach(), torch.ones_like(delta))
         tangent = torch.autograd.forward_ad.unpack_dual(compress.sparsegpt_2_4(dual, 4, H.detach())[0]).tangent
         assert tangent is None or not tangent.any()
+
+
+def fed_back(W, E, U):
+    from deltazip_b200 import compress
+    (n, count), c = E.shape, U.shape[1]
+    wide = torch.zeros((n, c + 8), device="cuda")
+    later = wide[:, 4:4 + c].copy_(W)
+    room = [torch.full((6 * s * count,), 3.0, dtype=torch.bfloat16, device="cuda") for s in (n, c)]
+    compress._feed_back(later, E.cuda(), U.cuda(), *room)
+    assert not wide[:, :4].any() and not wide[:, 4 + c:].any()
+    return later.double().cpu()
+
+
+@pytest.mark.parametrize("n,count,c", [(1, 4, 4), (33, 60, 100), (512, 128, 1028)])
+def test_update_of_the_columns_behind(n, count, c):
+    g = torch.Generator().manual_seed(n + c)
+    W, E, U = (torch.randn(s, generator=g) * f for s, f in (((n, c), 1e-3), ((n, count), 1e-4), ((count, c), 1.0)))
+    want, size = W.double() - E.double() @ U.double(), E.double().abs() @ U.double().abs()
+    error = (fed_back(W, E, U) - want).abs()
+    # what the split leaves out, and sums of 6 count terms in 32 bits that may be cut
+    assert (error <= (2.0 ** -23 + 6 * count * 2.0 ** -23) * size + 2.0 ** -23 * W.abs()).all()
+    if n == 512:                                   # in all no further off than a product in 32 bits
+        plain = torch.addmm(W.cuda(), E.cuda(), U.cuda(), alpha=-1).double().cpu()
+        assert error.norm() <= (plain - want).norm()
+
+
+@pytest.mark.parametrize("size", [2.0 ** -60, 2.0 ** -70, 2.0 ** -112, 2.0 ** -120, 2.0 ** 25, 2.0 ** 34, 2.0 ** 100])
+def test_update_by_errors_of_any_size(size):
+    """A third bf16 part has no bits left below 2^-109; the update is one of 32 bits at all sizes."""
+    n, count, c = 9, 128, 132
+    g = torch.Generator().manual_seed(0)
+    W, E, U = (torch.randn(s, generator=g) * f for s, f in (((n, c), size), ((n, count), size), ((count, c), 1.0)))
+    E[3:5] = torch.randn((2, count), generator=g)      # (rows of another size, and one of zeros)
+    E[7] = 0
+    got, want = fed_back(W, E, U), W.double() - E.double() @ U.double()
+    # sums of `count` rounded terms, or of 6 count terms that may be cut where the sizes are those of the tensor cores
+    terms = torch.full((n, 1), count * 0.5 if abs(np.log2(size)) > 64 or size > 2 ** 32 else 6.0 * count, dtype=torch.float64)
+    terms[3:5] = 6.0 * count
+    room = (E.double().abs() @ U.double().abs()) * 2.0 ** -23 * (terms + 1) + 2.0 ** -23 * W.abs() + 2.0 ** -148
+    assert ((got - want).abs() <= room).all()
+    assert torch.equal(got[7], W[7].double())
+
+
+def test_update_by_errors_that_are_not_finite():
+    n, count, c = 6, 8, 12
+    W, E, U = torch.zeros((n, c)), torch.ones((n, count)), torch.ones((count, c)) * (1 + 2.0 ** -20)
+    U[1] = 2.0 ** -40
+    E[1, 2], E[2, 1], E[3, 0], E[4, 5] = float("inf"), float("-inf"), float("nan"), 3.4e38
+    got = fed_back(W, E, U)
+    assert (got[1] == float("-inf")).all() and (got[2] == float("inf")).all() and got[3].isnan().all()
+    assert torch.allclose(got[4], torch.full((c,), -3.4e38, dtype=torch.float64) * (1 + 2.0 ** -20), rtol=2.0 ** -22)
+    assert torch.allclose(got[[0, 5]], -(E.double() @ U.double())[[0, 5]], rtol=2.0 ** -20)
