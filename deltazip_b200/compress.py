@@ -190,6 +190,8 @@ def sparsegpt_2_4(delta: torch.Tensor, bits: int, H: Optional[torch.Tensor] = No
         hinv, dead = hinv_factor(H.to(W.device, torch.float32), percdamp)
         W[:, dead] = 0
     else:
+        if hinv.shape != (k, k):
+            raise ValueError(f"hinv must be [{k}, {k}]")
         hinv = hinv.to(W.device, torch.float32).contiguous()
     loss = torch.zeros(n, dtype=torch.float32, device=W.device)
     L, factor = lib(), hinv.detach()

@@ -197,3 +197,10 @@ def test_update_by_errors_that_are_not_finite():
     assert (got[1] == float("-inf")).all() and (got[2] == float("inf")).all() and got[3].isnan().all()
     assert torch.allclose(got[4], torch.full((c,), -3.4e38, dtype=torch.float64) * (1 + 2.0 ** -20), rtol=2.0 ** -22)
     assert torch.allclose(got[[0, 5]], -(E.double() @ U.double())[[0, 5]], rtol=2.0 ** -20)
+
+
+@pytest.mark.parametrize("shape", [(128, 128), (256, 128), (512, 512), (256,)])
+def test_a_factor_of_another_size_is_refused(shape):
+    from deltazip_b200 import compress
+    with pytest.raises(ValueError, match="256, 256"):
+        compress.sparsegpt_2_4(torch.zeros((8, 256), device="cuda"), 4, hinv=torch.ones(shape, device="cuda"))
