@@ -5,8 +5,9 @@ Follows deltazip/core/sparsegpt.py (`SparseGPT.add_batch` :25-43, `fasterprune` 
 prunen:prunem = 2:4, no activation ordering) and `QuantLinear.pack`
 (deltazip/nn_modules/qlinear.py:83-183).  The per-column loop of a block -- mask, quantise,
 propagate the error inside the block -- is one kernel launch per 128 columns (dz_sparsegpt_block_strided,
-rows in parallel); the dense linear algebra around it (the Cholesky factorisation of H, the
-rank-128 update of the columns behind a block) are library calls, as in the reference.
+rows in parallel); the dense linear algebra around it (the Cholesky factorisation of H, the products that
+join the inverse's blocks, the rank-128 update of the columns behind a block) are library calls on operands
+that kernels here prepare.
 """
 from __future__ import annotations
 

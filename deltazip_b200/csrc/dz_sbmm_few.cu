@@ -396,25 +396,26 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) sbmm_few_kernel(const 
 // features), and not too much delta work.  A CTA's warps go through all of k, delta by delta, where the larger form splits k
 // over CTAs and hands the products to tcgen05.mma.sp: k times deltas (at most min(tokens, slots)) is the chain here, the
 // whole delta work the chip's load, and twice the columns make both twice as long.  With one slice an SM the chain has the
-// SM to itself and may be longer.  Times in us, larger form against this one, fp16 4-bit, weights and slots not in L2, device
-// time in a graph (2-bit codes and bf16 lie on the same side):
+// SM to itself and may be longer; at equal times this form is the better one, as its launch encodes no tensor maps.  Times in
+// us, larger form against this one, fp16 4-bit, weights and slots not in L2, device time in a graph (2-bit codes and bf16 lie
+// on the same side):
 //   base product alone    1 row   4096 x 4096 17.1, 8.6   12288 x 4096 35.4, 18.8   22016 x 4096 40.4, 30.9   32000 x 4096 55.4, 41.5
 //                         16 rows             17.5, 10.2              36.1, 20.8               40.9, 35.1               56.7, 46.2
 //   8 tokens, by deltas   11264 x 2048 3: 20.5, 17.8 (4: 22.1, 21.1; 6: 25.4, 28.7)    6144 x 2048 4: 15.4, 14.5 (6: 17.7, 19.1)
 //                         4096 x 4096 2: 16.3, 15.1 (3: 17.0, 16.9; 4: 18.0, 19.2)     12288 x 4096 1: 29.8, 25.6 (4: 36.9, 37.5)
 //                         5120 x 5120 1: 19.5, 17.3 (2: 20.5, 21.3)     22016 x 4096 (1: 46.1, 45.7; 2: 49.3, 53.4)
-//     one slice an SM     2048 x 2048 8: 13.3, 11.7    1024 x 4096 4: 13.5, 12.9 (6: 14.5, 16.7)    2048 x 5632 2: 14.7, 14.0 (4: 15.6, 16.9)
+//     one slice an SM     2048 x 2048 8: 13.3, 11.7    1024 x 4096 4: 13.5, 12.9 (6: 14.5, 16.7)    2048 x 5632 3: 15.1, 15.1 (4: 15.6, 16.9)
 //                         1024 x 6144 1: 13.9, 12.6 (but 1280 x 8192 1: 14.6, 15.8)
 //   16 tokens             2048 x 2048 4: 11.9, 10.3 (8: 13.3, 13.5)     4096 x 4096 1: 15.7, 15.6 (2: 16.2, 18.4)
 //                         1024 x 4096 2: 13.1, 12.8 (3: 13.3, 13.7)     2048 x 5632 1: 14.4, 14.2 (but 1024 x 6144 1: 13.9, 14.7)
-// Of 1592 measured calls on this side of the line seven are faster in the larger form, by 3 % at most (1024 x 6144, 2 deltas);
+// Of 1596 measured calls on this side of the line seven are faster in the larger form, by 3 % at most (1024 x 6144, 2 deltas);
 // by the product of deltas and weights alone 1280 x 8192 with 6 deltas took 29.4 where the larger form takes 17.9.
 bool sbmm_few_supported(const dz_sbmm_args& a, bool base_only, int sms) {
   if (a.M > kFewMax || a.push) return false;
   if (base_only) return true;
   const long long deltas = min(a.M, a.num_slots), chain = deltas * a.K, work = chain * a.N;
   if (a.M > 8) return a.K <= 5632 && chain <= 8192 && work <= 1ll << 24;
-  return a.K <= 6144 && chain <= (a.N / 16 <= sms ? 16384 : 8192) && work <= 70000000ll;
+  return a.K <= 6144 && chain <= (a.N / 16 <= sms ? 17000 : 8192) && work <= 70000000ll;
 }
 
 int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status, cudaStream_t st) {
@@ -438,8 +439,8 @@ int launch_sbmm_few(const dz_sbmm_args& a, bool base_only, int sms, int* status,
   static const Kern kerns[24] = {DZ_FEW(1, 1, 8), DZ_FEW(2, 1, 8), DZ_FEW(1, 2, 8), DZ_FEW(2, 2, 8), DZ_FEW(1, 2, 4), DZ_FEW(2, 2, 4)};
 #undef DZ_FEW
   // Slices of 32 features, with half the work per delta that does not grow with the features (metadata, masking x), where
-  // two CTAs an SM have one each; narrower ones keep more SMs busy (one token, one delta: 4096 x 4096 10.3 us with 16, 11.1
-  // with 32; 12288 x 4096 31.2 and 24.4).  Two CTAs of eight warps an SM; four of four where the slices are more than those.
+  // two CTAs an SM have one each; narrower ones keep more SMs busy (one token, one delta: 2048 x 2048 6.7 us with 16, 7.1
+  // with 32; 4096 x 4096 12.8 and 12.3; 6144 x 2048 13.3 and 9.4; 12288 x 4096 32.1 and 25.9).  Two CTAs of eight warps an SM; four of four where the slices are more than those.
   const int rt = a.N / 16 > 2 * sms ? 2 : 1, slices = a.N / (16 * rt), warps = slices > 2 * sms ? 4 : 8;
   // Three of those, held down to that by their shared memory, where rounds of three end sooner than rounds of four: with
   // four some SMs get four CTAs and others two.  Base products of 9 rows, three always (four did not fit) and so: 11264 x

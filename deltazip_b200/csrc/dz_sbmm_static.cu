@@ -81,7 +81,7 @@ extern "C" int dz_sbmm_static(const dz_sbmm_args* args, void* stream) {
   if (rc) return rc;
 
   cudaStream_t st = (cudaStream_t)stream;
-  // the tile counters must start at zero; the status word before them is left alone
+  // the tile counters must start at zero (few tokens use none); the status word before them is left alone
   DZ_CUDA_OK(cudaMemsetAsync(static_cast<unsigned char*>(scratch) + kWsCounters, 0,
                              kWsCountersBytes, st));
   dz_sbmm_args a = *args;

@@ -1078,7 +1078,7 @@ DeviceInfo& device_info(int dev) {
 size_t sbmm_workspace_bytes(int M, int N, int K, int tokens_sorted) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   size_t b = kWsPartials + sbmm_partial_bytes(M);
-  if (!tokens_sorted) b += (size_t)round_up(M, 16) * K * 2 + 1024;
+  if (!tokens_sorted) b += (size_t)round_up(M, 16) * K * 2 + 1024;   // (also for rows that are not gathered: as ever)
   return b;
 }
 

@@ -135,8 +135,9 @@ class Segments:
         `sorted_hint=True` is the caller's promise that `indices` is non-decreasing (the
         reference's scheduler delivers batches sorted by delta id,
         serving/vllm/core/scheduler.py:101-104): x is then read in place.  Without the
-        promise the SBMM first gathers x into sorted order on the device (a plain copy when
-        the batch happens to be sorted), so any order is handled."""
+        promise the SBMM first gathers more than 16 rows of x into sorted order on the device
+        (a plain copy when the batch happens to be sorted) and takes fewer as they come, so
+        any order is handled."""
         _need_cuda(indices)
         m = indices.numel()
         if m > self.max_tokens:
@@ -383,8 +384,9 @@ def _segments_for(indices: torch.Tensor, num_slots: int, device) -> Segments:
     (the `copy_` of the reference's _set_delta_mapping, serving/vllm/delta/models.py:407-430)
     advances.  The cache keeps the tensor alive, so the address cannot be handed to another
     tensor while the entry exists.  All layers of a step therefore share one build, with no
-    host synchronisation: whether the batch is sorted is left to the device (x is gathered
-    through the table's permutation, which is the identity for a sorted batch)."""
+    host synchronisation: whether the batch is sorted is left to the device (more than 16
+    rows of x are gathered through the table's permutation, which is the identity for a sorted
+    batch; fewer are taken in their own order)."""
     indices = indices.reshape(-1)
     m = indices.numel()
     key = (device.index, _stream(), num_slots)

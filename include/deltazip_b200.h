@@ -138,10 +138,12 @@ typedef struct {
   int32_t tokens_sorted;    /* 1: caller guarantees `indices` were non-decreasing
                                (the reference's scheduler sorts each batch by
                                delta id, serving/vllm/core/scheduler.py:101-104);
-                               x is then read in place.  0: no promise -- x is
-                               first gathered into sorted order inside the
-                               workspace (a plain copy when the batch happens to
-                               be sorted); no host synchronisation either way.
+                               x is then read in place.  0: no promise -- more
+                               than 16 rows of x are first gathered into sorted
+                               order inside the workspace (a plain copy when the
+                               batch happens to be sorted), fewer are taken in
+                               their own order (the workspace is demanded all the
+                               same); no host synchronisation either way.
                                A wrong promise is detected (DZ_ERR_INVALID_ARG in
                                the workspace status word) and nothing is computed. */
   int32_t flags;            /* DZ_SBMM_* bits, 0 = none                          */

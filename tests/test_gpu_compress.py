@@ -140,7 +140,7 @@ def _columns_one_by_one(delta, hinv, scale, zero, bits):
 @pytest.mark.parametrize("bits", [2, 4])
 @pytest.mark.parametrize("k", [512, 516, 640, 1100])
 def test_error_feedback_across_spans_of_blocks(k, bits):
-    """Columns behind a span of four blocks are updated once for the span, those within it per block.  A decision that
+    """The columns behind a block of 128 are updated by its errors at once, block after block.  A decision that
     rounding turns (a weight within 2^-24 x K of a boundary: fewer than one row here) changes the rest of its row: at most
     two of 64 rows may differ; a block without its update changes them all."""
     from deltazip_b200 import compress

@@ -72,6 +72,23 @@ def test_one_block(n, count, lead, size):
         assert (np.abs(loss - true) <= (count + 4) * 2.0 ** -23 * true + 1e-37).all()
 
 
+@pytest.mark.parametrize("n,count", [(5, 128), (33, 36)])
+def test_one_block_into_matrices_of_its_own(n, count):
+    """dz_sparsegpt_block: rows of the results `count` apart, the block left as it was."""
+    from deltazip_b200._lib import check, lib
+    rng = np.random.default_rng(n)
+    W = rng.standard_normal((n, count)).astype(F)
+    h = (np.triu(rng.standard_normal((count, count)) * 0.2, 1) + np.diag(0.5 + rng.random(count))).astype(F)
+    scale, zero = (np.abs(W).max(1) * F(2 / 15)).astype(F), np.full(n, 8, F)
+    w, H, s, z = (torch.from_numpy(a).cuda() for a in (W, h, scale, zero))
+    Q, E = torch.empty((n, count), device="cuda"), torch.empty((n, count), device="cuda")
+    check(lib().dz_sparsegpt_block(w.data_ptr(), count, H.data_ptr(), count, s.data_ptr(), z.data_ptr(), 4, n, count,
+                                   Q.data_ptr(), E.data_ptr(), None, torch.cuda.current_stream().cuda_stream), "block")
+    want_q, want_e = one_block(W, h, scale, zero, 15)
+    assert np.array_equal(Q.cpu().numpy(), want_q) and np.array_equal(E.cpu().numpy(), want_e)
+    assert np.array_equal(w.cpu().numpy(), W)
+
+
 @pytest.mark.parametrize("k", [1, 7, 128, 129, 300, 512])
 def test_inverses_of_diagonal_blocks(k):
     from deltazip_b200._lib import check, lib
